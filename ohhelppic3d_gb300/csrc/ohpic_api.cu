@@ -29,35 +29,84 @@ int fail(ohpic_ctx *c, int code, const std::string &msg)
 
 int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
-// Largest power-of-two tile edge <= 8 that divides n.
-int default_tile(int n)
+// Default tile edge of an axis of n cells: the axis in equal tiles of about
+// `want` cells (at most want + 2), tiles that divide it preferred.  The last tile
+// of an axis that does not divide may be shorter.
+int default_edge(int n, int want)
 {
-    for (int t = 8; t > 1; t >>= 1)
-        if (n % t == 0) return t;
-    return 1;
+    if (n <= want + 2 && n < 2 * want - want / 2) return n;
+    int best = want, best_cost = INT32_MAX;
+    for (int nt = std::max(1, n / want); nt <= n / want + 1; ++nt) {
+        const int t = (n + nt - 1) / nt;
+        if (t > want + 2) continue;
+        const int cost = 2 * std::abs(t - want) + (n % t ? 3 : 0);
+        if (cost < best_cost) {
+            best = t;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+int64_t tiles_of(const int n[3], const int tile[3])
+{
+    int64_t nt = 1;
+    for (int d = 0; d < 3; ++d) nt *= (n[d] + tile[d] - 1) / tile[d];
+    return nt;
+}
+
+// Default tile of a grid: edges of about 8 cells, or of about 4 along z, then y,
+// then x while the species' tiles are too few to occupy the chip (152 SMs, two
+// CTAs each).  FP32 push, tiles of 8 x 8 x 8 against the ones this rule takes,
+// both with one CTA per tile: 16^3 x 8 ppc 35 -> 15.8 us (4 x 4 x 4), 24^3 x 16
+// ppc 49 -> 26 us (8 x 4 x 4), 32^3 x 16 ppc 49.6 -> 37.9 us (8 x 8 x 4); FP64 at
+// 32^3 353 -> 249 us.  From 48^3 on (432 tiles) 8 x 8 x 8 is as fast as any.
+// Two CTAs must fit an SM (boxes of at most kPairNodes nodes).
+constexpr int64_t kFewTiles = 200;
+
+void default_tile(const ohpic_config &k, int halo, int tile[3])
+{
+    const int n[3] = {k.nx, k.ny, k.nz};
+    const int64_t pair_nodes = k.precision == OHPIC_FP64 ? 2880 : 3540;
+    int want[3] = {8, 8, 8};
+    for (int d = 0; d < 3; ++d) tile[d] = k.tile[d] > 0 ? k.tile[d] : default_edge(n[d], want[d]);
+    for (int d = 2; d >= 0 && k.nspecies * tiles_of(n, tile) < kFewTiles; --d) {
+        want[d] = 4;
+        if (k.tile[d] <= 0) tile[d] = default_edge(n[d], want[d]);
+    }
+    auto nodes = [&]() {
+        int64_t v = 1;
+        for (int d = 0; d < 3; ++d) v *= tile[d] + 2 * halo + 1;
+        return v;
+    };
+    for (int d = 2; d >= 0 && nodes() > pair_nodes; --d)
+        if (k.tile[d] <= 0) tile[d] = std::min(tile[d], want[d]);
 }
 
 }  // namespace
 
 namespace ohpic {
 
-// Grid geometry for a tile shape and halo; false when a tile edge is not a
-// divisor of the grid or the staged box does not fit one CTA's shared memory.
-bool make_geom(const ohpic_config &k, const int tile[3], int halo, Geom &g)
+// Grid geometry for a tile shape and halo; false when a tile edge neither
+// divides the grid nor is the axis' default edge (given by default_of), or the
+// staged box does not fit one CTA's shared memory.
+bool make_geom(const ohpic_config &k, const int tile[3], int halo, Geom &g, const int *default_of)
 {
     const int n[3] = {k.nx, k.ny, k.nz};
     for (int d = 0; d < 3; ++d)
-        if (tile[d] < 1 || tile[d] > 64 || n[d] % tile[d] != 0) return false;
+        if (tile[d] < 1 || tile[d] > 64 || (n[d] % tile[d] != 0 && !(default_of && tile[d] == default_of[d])))
+            return false;
     if (halo < 0 || halo > kMaxHalo) return false;
     g.nx = k.nx; g.ny = k.ny; g.nz = k.nz;
     g.tx = tile[0]; g.ty = tile[1]; g.tz = tile[2];
-    g.ntx = g.nx / g.tx; g.nty = g.ny / g.ty; g.ntz = g.nz / g.tz;
+    g.ntx = (g.nx + g.tx - 1) / g.tx; g.nty = (g.ny + g.ty - 1) / g.ty; g.ntz = (g.nz + g.tz - 1) / g.tz;
     g.halo = halo;
     g.sx = g.tx + 2 * halo + 1; g.sy = g.ty + 2 * halo + 1; g.sz = g.tz + 2 * halo + 1;
     g.gx = g.nx + 2 * halo + 1; g.gy = g.ny + 2 * halo + 1; g.gz = g.nz + 2 * halo + 1;
     g.ncell = (int64_t)g.nx * g.ny * g.nz;
     g.ntile = (int64_t)g.ntx * g.nty * g.ntz;
     g.tile_cells = g.tx * g.ty * g.tz;
+    g.nkeys = g.ntile * g.tile_cells;
     g.nxh = g.nx / 2 + 1;
     g.nspec = (int64_t)g.nxh * g.ny * g.nz;
     // Staged E box (4 reals per node) plus the deposit box (8 bytes per node).
@@ -357,11 +406,11 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
         if (k.capacity[s] < 0 || k.capacity[s] > (int64_t)UINT32_MAX) return OHPIC_ERR_INVALID;
         if (!(k.qm[s] != 0.0) || !std::isfinite(k.qm[s]) || !std::isfinite(k.q[s])) return OHPIC_ERR_INVALID;
     }
-    const int tile[3] = {k.tile[0] > 0 ? k.tile[0] : default_tile(k.nx), k.tile[1] > 0 ? k.tile[1] : default_tile(k.ny),
-                         k.tile[2] > 0 ? k.tile[2] : default_tile(k.nz)};
     const int n[3] = {k.nx, k.ny, k.nz};
     for (int d = 0; d < 3; ++d)
-        if (n[d] % tile[d] != 0 || tile[d] > 64) return OHPIC_ERR_INVALID;
+        if (k.tile[d] > 0 && (n[d] % k.tile[d] != 0 || k.tile[d] > 64)) return OHPIC_ERR_INVALID;
+    int tile[3];
+    default_tile(k, 2, tile);
 
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || k.device < 0 || k.device >= ndev) {
@@ -387,10 +436,14 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     c->sort_lead = 0;
     c->tma_polls = kTmaWaitPolls;
     Geom &g = c->g;
-    if (!make_geom(k, tile, c->halo, g)) {
+    for (int d = 0; d < 3; ++d) c->def_tile[d] = tile[d];
+    if (!make_geom(k, tile, c->halo, g, c->def_tile)) {
         ohpic_destroy(c);
         return OHPIC_ERR_INVALID;
     }
+    // sort keys of any tile this context accepts: a tile edge divides its axis or
+    // is the default one, whose tiles cover at least the axis
+    const int64_t nkeys = std::max(g.nkeys, g.ncell);
 
     int64_t off = 0;
     for (int s = 0; s < k.nspecies; ++s) {
@@ -428,10 +481,10 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     if (rc == OHPIC_OK) rc = dalloc(c, (char **)&c->epad, (int64_t)g.gx * g.gy * g.gz * 4 * es);
     if (rc == OHPIC_OK) rc = dalloc(c, (char **)&c->spec, g.nspec * 2 * es);
     if (rc == OHPIC_OK) rc = dalloc(c, &c->green, g.nspec);
-    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_count, g.ncell);
-    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_stay, g.ncell);
-    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_start, g.ncell + 1);
-    if (rc == OHPIC_OK) rc = dalloc(c, &c->scan_tmp, scan_tmp_elems(g.ncell));
+    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_count, nkeys);
+    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_stay, nkeys);
+    if (rc == OHPIC_OK) rc = dalloc(c, &c->cell_start, nkeys + 1);
+    if (rc == OHPIC_OK) rc = dalloc(c, &c->scan_tmp, scan_tmp_elems(nkeys));
     if (rc == OHPIC_OK) rc = dalloc(c, &c->key_table, (int64_t)g.nx + g.ny + g.nz);
     if (rc == OHPIC_OK) rc = dalloc(c, &c->tile_begin, (int64_t)k.nspecies * (g.ntile + 1));
     if (rc == OHPIC_OK) {
@@ -901,7 +954,7 @@ int ohpic_set_tuning(ohpic_ctx *c, const ohpic_tuning *t)
     if (t->sort_lead < 0 || t->sort_lead > 4096 || (t->sort_lead != 0 && c->cfg.precision != OHPIC_FP32))
         return fail(c, OHPIC_ERR_INVALID, "tuning: sort_lead 0..4096, nonzero only in the FP32 form");
     Geom g2;
-    if (!make_geom(c->cfg, t->tile, t->halo, g2))
+    if (!make_geom(c->cfg, t->tile, t->halo, g2, c->def_tile))
         return fail(c, OHPIC_ERR_INVALID, "tuning: tile edges must divide the grid (<= 64) and the staged box fit");
     cudaSetDevice(c->dev);
     materialize_records(c);

@@ -53,7 +53,7 @@ __host__ __device__ inline int cell_z(int32_t c) { return (int)((uint32_t)c >> (
 // Grid geometry shared by every kernel (passed by value).
 struct Geom {
     int nx, ny, nz;
-    int tx, ty, tz;        // tile shape (cells); power-of-two divisors of n
+    int tx, ty, tz;        // tile shape (cells); divisors of n, or the default edges (last tile shorter)
     int ntx, nty, ntz;     // tiles per axis
     int halo;              // cells staged around a tile
     int sx, sy, sz;        // staged nodes per axis: t + 2*halo + 1
@@ -61,6 +61,7 @@ struct Geom {
     int64_t ncell;
     int64_t ntile;
     int tile_cells;
+    int64_t nkeys;         // sort keys: ntile * tile_cells (>= ncell; more when the last tiles are shorter)
     int nxh;               // nx/2 + 1
     int64_t nspec;         // nz*ny*nxh
 };
@@ -266,6 +267,7 @@ struct ohpic_ctx {
     bool field_valid;
     int64_t steps;
     int split;
+    int def_tile[3];            // tile the context was created with
     int halo;
     int dep_strategy;           // OHPIC_DEPOSIT_* for the FP32 warp deposit
     int lane_particles;         // FP32 push/deposit: particles per lane (2 or 4)
@@ -288,7 +290,7 @@ namespace ohpic {
 
 // Host helpers (ohpic_api.cu): geometry of a grid for a tile shape and halo
 // (false when it does not fit), and the FP64 Boris constants of one species.
-bool make_geom(const ohpic_config &k, const int tile[3], int halo, Geom &g);
+bool make_geom(const ohpic_config &k, const int tile[3], int halo, Geom &g, const int *default_of = nullptr);
 void species_consts(const ohpic_config &cfg, int s, double dt, SpeciesConst &k);
 
 // Kernel launchers: dispatch (convert.cu) and the two forms (push_f64.cu, push_f32.cu).

@@ -242,9 +242,11 @@ __device__ __forceinline__ void stage_f32(const TileArgs &a, const Item &it, flo
         for (int r = threadIdx.x >> 5; r < rows; r += nw) {
             const int cz = r / g.sy, by = r - cz * g.sy;
             // padded index of node x0 - halo + ax is x0 + ax
+            // (the box of a shorter last tile reaches past the array)
+            if (it.z0 + cz >= g.gz || it.y0 + by >= g.gy) continue;
             const float4 *src = E + ((int64_t)(it.z0 + cz) * g.gy + (it.y0 + by)) * g.gx + it.x0;
-            const int base = r * g.sx;
-            for (int ax = lane; ax < g.sx; ax += 32) sE[base + ax] = __ldg(src + ax);
+            const int base = r * g.sx, ex = min(g.sx, g.gx - it.x0);
+            for (int ax = lane; ax < ex; ax += 32) sE[base + ax] = __ldg(src + ax);
         }
     }
     if (need_w) {

@@ -814,7 +814,7 @@ static void sort_tiles(ohpic_ctx *c, float h)
     for (int s = 0; s < c->cfg.nspecies; ++s) {
         const int64_t n = c->count[s];
         int64_t *tb = c->tile_begin + (int64_t)s * (g.ntile + 1);
-        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.ncell, c->stream);
+        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.nkeys, c->stream);
         if (f32 && h != 0.f)
             k_hist_tile<true, true><<<(unsigned)g.ntile, 256, smem, c->stream>>>(
                 g, c->key_table, c->p64[src], c->p32[src], tb, c->cell_stay, c->cell_count, h, c->diag);
@@ -827,8 +827,8 @@ static void sort_tiles(ohpic_ctx *c, float h)
                                                                            tb, c->cell_stay, c->cell_count, 0.f,
                                                                            c->diag);
         ++c->launches;
-        scan_exclusive(c, c->cell_stay, c->cell_start, g.ncell, c->scan_tmp, c->cell_count);
-        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.ncell, c->stream);
+        scan_exclusive(c, c->cell_stay, c->cell_start, g.nkeys, c->scan_tmp, c->cell_count);
+        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.nkeys, c->stream);
         if (f32) {
             k_scatter_tile<true><<<(unsigned)g.ntile, 256, smem, c->stream>>>(
                 g, c->key_table, c->p64[src], c->p32[src], c->ids[src], c->pblock[dst], tb, c->seg[s], c->cell_start,
@@ -872,7 +872,7 @@ int sort_particles(ohpic_ctx *c)
     for (int s = 0; s < c->cfg.nspecies; ++s) {
         const int64_t n = c->count[s];
         int64_t *tb = c->tile_begin + (int64_t)s * (g.ntile + 1);
-        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.ncell, c->stream);
+        cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.nkeys, c->stream);
         if (n > 0) {
             if (f32)
                 if (h != 0.f)
@@ -887,12 +887,12 @@ int sort_particles(ohpic_ctx *c)
                                                                  c->seg[s], n, c->cell_count, 0.f, c->diag);
             ++c->launches;
         }
-        scan_exclusive(c, c->cell_count, c->cell_start, g.ncell, c->scan_tmp);
+        scan_exclusive(c, c->cell_count, c->cell_start, g.nkeys, c->scan_tmp);
         k_tile_begin<<<(unsigned)((g.ntile + 1 + 255) / 256), 256, 0, c->stream>>>(g, c->cell_start, c->seg[s], n,
                                                                                     tb);
         ++c->launches;
         if (n > 0) {
-            cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.ncell, c->stream);
+            cudaMemsetAsync(c->cell_count, 0, sizeof(uint32_t) * g.nkeys, c->stream);
             // records in the other buffer's block, then back into this buffer:
             // FP32 by the next push (or materialize_records), FP64 here
             if (f32) {

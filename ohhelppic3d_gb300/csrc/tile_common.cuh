@@ -209,8 +209,10 @@ __device__ __forceinline__ void stage_tile(const TileArgs &a, const Item &it, No
     for (int i = threadIdx.x; i < s3; i += blockDim.x) {
         if (need_e) {
             const int ax = i % g.sx, by = (i / g.sx) % g.sy, cz = i / (g.sx * g.sy);
-            // padded index of node (x0 - halo + ax) is x0 + ax
-            sE[i] = ldg_node(E + ((int64_t)(it.z0 + cz) * g.gy + (it.y0 + by)) * g.gx + (it.x0 + ax));
+            // padded index of node (x0 - halo + ax) is x0 + ax; the box of a last tile
+            // that is shorter than the others reaches past the array
+            if (it.x0 + ax < g.gx && it.y0 + by < g.gy && it.z0 + cz < g.gz)
+                sE[i] = ldg_node(E + ((int64_t)(it.z0 + cz) * g.gy + (it.y0 + by)) * g.gx + (it.x0 + ax));
         }
         if (need_rho) srho[i] = T(0);
     }
