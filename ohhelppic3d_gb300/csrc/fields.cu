@@ -17,6 +17,7 @@
 #include <cufft.h>
 #include <stdint.h>
 
+#include "field_nodes.cuh"
 #include "ohpic_internal.cuh"
 
 namespace ohpic {
@@ -72,181 +73,6 @@ __global__ void k_scale_c(cufftComplex *spec, const double *green, int64_t n)
     }
 }
 
-__device__ __forceinline__ int wrapn(int i, int n)
-{
-    i %= n;
-    return i < 0 ? i + n : i;
-}
-
-// Padded E node t from phi (n^3), periodic ghosts included.
-template <typename T, typename NodeT>
-__device__ __forceinline__ void stencil_node(const Geom &g, const T *phi, NodeT *epad, int64_t t)
-{
-    const int64_t nxy = (int64_t)g.nx * g.ny;
-    {
-        const int px = (int)(t % g.gx);
-        const int py = (int)((t / g.gx) % g.gy);
-        const int pz = (int)(t / ((int64_t)g.gx * g.gy));
-        const int i = wrapn(px - g.halo, g.nx), j = wrapn(py - g.halo, g.ny), k = wrapn(pz - g.halo, g.nz);
-        const int im = i == 0 ? g.nx - 1 : i - 1, ip = i + 1 == g.nx ? 0 : i + 1;
-        const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j + 1 == g.ny ? 0 : j + 1;
-        const int km = k == 0 ? g.nz - 1 : k - 1, kp = k + 1 == g.nz ? 0 : k + 1;
-        const int64_t row = (int64_t)j * g.nx + (int64_t)k * nxy;
-        const T p0 = phi[i + row];
-        NodeT e;
-        e.x = T(0.5) * ((phi[im + row] - p0) + (p0 - phi[ip + row]));
-        e.y = T(0.5) * ((phi[i + (int64_t)jm * g.nx + (int64_t)k * nxy] - p0) +
-                        (p0 - phi[i + (int64_t)jp * g.nx + (int64_t)k * nxy]));
-        e.z = T(0.5) * ((phi[i + row - (int64_t)k * nxy + (int64_t)km * nxy] - p0) +
-                        (p0 - phi[i + row - (int64_t)k * nxy + (int64_t)kp * nxy]));
-        e.w = T(0);
-        epad[t] = e;
-    }
-}
-
-template <typename T, typename NodeT>
-__global__ void k_stencil(Geom g, const T *phi, NodeT *epad)
-{
-    const int64_t total = (int64_t)g.gx * g.gy * g.gz;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
-        stencil_node<T, NodeT>(g, phi, epad, t);
-}
-
-// ---- FP32 form: rho from the fixed-point weight sums ----
-//
-// rho = sum_s q_s * W_s * 2^-24 (W_s the species' integer weight sum at the
-// node), rounded once to FP32.  Each charge is an integer mantissa times a power
-// of two (from its bit pattern), so the sum is formed exactly in 128-bit integer
-// arithmetic and rounded to nearest, ties to even: no FP64 arithmetic per node.
-// Bounds: |m_s| < 2^53, W_s < 2^58 (every count is far below 2^34), the exponent
-// spread at most kRhoMaxShift, at most 8 species: the sum stays below 2^126.
-// Charges further apart in exponent (or subnormal), and sums outside the normal
-// FP32 range, take the FP64 expression instead.
-constexpr int kRhoMaxShift = 12;
-
-struct RhoScale {
-    long long m[OHPIC_MAX_SPECIES];
-    int shift[OHPIC_MAX_SPECIES];
-    int K;
-    bool ok;
-};
-
-__device__ __forceinline__ RhoScale rho_scale(const double *q, int nsp)
-{
-    RhoScale r;
-    r.ok = true;
-    r.K = 0x7fffffff;
-    int k[OHPIC_MAX_SPECIES];
-    for (int s = 0; s < nsp; ++s) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(q[s]);
-        const int e = (int)((b >> 52) & 0x7ffu);
-        const long long mant = (long long)(b & ((1ull << 52) - 1));
-        r.m[s] = 0;
-        k[s] = 0;
-        if (e == 0) {
-            if (mant != 0) r.ok = false;   // subnormal charge
-            continue;
-        }
-        if (e == 0x7ff) {
-            r.ok = false;
-            continue;
-        }
-        const long long m = mant | (1ll << 52);
-        r.m[s] = (b >> 63) ? -m : m;
-        k[s] = e - 1075 - 24;              // q_s * 2^-24 = m * 2^k
-        r.K = min(r.K, k[s]);
-    }
-    for (int s = 0; s < nsp; ++s) {
-        r.shift[s] = r.m[s] != 0 ? k[s] - r.K : 0;
-        if (r.shift[s] > kRhoMaxShift) r.ok = false;
-    }
-    if (r.K == 0x7fffffff) r.K = 0;        // every charge zero: the sum is 0
-    return r;
-}
-
-// acc * 2^K rounded to FP32, nearest with ties to even; false outside the
-// normal range.
-__device__ __forceinline__ bool i128_to_float_rne(__int128 acc, int K, float &out)
-{
-    if (acc == 0) {
-        out = 0.f;
-        return true;
-    }
-    const bool neg = acc < 0;
-    const unsigned __int128 a = neg ? (unsigned __int128)(-acc) : (unsigned __int128)acc;
-    const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-    int msb = hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)lo);
-    unsigned int mant;
-    if (msb <= 23) {
-        mant = (unsigned int)(lo << (23 - msb));
-    } else {
-        const int sh = msb - 23;
-        const unsigned __int128 one = 1;
-        const unsigned __int128 rem = a & ((one << sh) - 1);
-        const unsigned __int128 half = one << (sh - 1);
-        mant = (unsigned int)(a >> sh);
-        if (rem > half || (rem == half && (mant & 1u))) {
-            ++mant;
-            if (mant == (1u << 24)) {
-                mant >>= 1;
-                ++msb;
-            }
-        }
-    }
-    const int be = msb + K + 127;
-    if (be < 1 || be > 254) return false;
-    out = __uint_as_float((neg ? 0x80000000u : 0u) | ((unsigned)be << 23) | (mant & 0x7fffffu));
-    return true;
-}
-
-// rho at one node: w[s * stride] is species s's weight sum.
-__device__ __forceinline__ float node_rho(const unsigned long long *w, int64_t stride, int nsp, const double *q,
-                                          const RhoScale &r)
-{
-    if (r.ok) {
-        __int128 acc = 0;
-        for (int s = 0; s < nsp; ++s) {
-            const long long m = r.m[s];
-            if (m == 0) continue;
-            // |m| * W as one 64 x 64 -> 128-bit product, then the species' shift
-            const unsigned long long W = w[s * stride];
-            const unsigned long long am = (unsigned long long)(m < 0 ? -m : m);
-            unsigned __int128 p = ((unsigned __int128)__umul64hi(am, W) << 64) | (unsigned __int128)(am * W);
-            p <<= r.shift[s];
-            acc = m < 0 ? acc - (__int128)p : acc + (__int128)p;
-        }
-        float v;
-        if (i128_to_float_rne(acc, r.K, v)) return v;
-    }
-    double acc = 0.0;
-    for (int s = 0; s < nsp; ++s) acc += q[s] * (double)w[s * stride];
-    return (float)(acc * kWeightUnit);
-}
-
-// node_rho of one or two species whose weight sums are already in registers.
-__device__ __forceinline__ float node_rho2(const unsigned long long W[2], int nsp, const double *q, const RhoScale &r)
-{
-    if (r.ok) {
-        __int128 acc = 0;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const long long m = s < nsp ? r.m[s] : 0;
-            if (m == 0) continue;
-            const unsigned long long am = (unsigned long long)(m < 0 ? -m : m);
-            unsigned __int128 p = ((unsigned __int128)__umul64hi(am, W[s]) << 64) | (unsigned __int128)(am * W[s]);
-            p <<= r.shift[s];
-            acc = m < 0 ? acc - (__int128)p : acc + (__int128)p;
-        }
-        float v;
-        if (i128_to_float_rne(acc, r.K, v)) return v;
-    }
-    double acc = 0.0;
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-        if (s < nsp) acc += q[s] * (double)W[s];
-    return (float)(acc * kWeightUnit);
-}
-
 // ---- pooled fields: many runs of one grid size, slot = blockIdx.y; on[slot] == 0 skips ----
 
 // rho of every active slot from its fixed-point weight sums (nsp species per slot,
@@ -280,17 +106,6 @@ __global__ void k_pool_scale(cufftComplex *spec, int64_t nspec, const double *gr
         v.y = (float)((double)v.y * gf);
         spec[i] = v;
     }
-}
-
-__global__ void k_pool_stencil(Geom g, const float *phi, float4 *epad, const int *on)
-{
-    const int slot = blockIdx.y;
-    if (on && !on[slot]) return;
-    const int64_t total = (int64_t)g.gx * g.gy * g.gz;
-    phi += (int64_t)slot * g.ncell;
-    epad += (int64_t)slot * total;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x)
-        stencil_node<float, float4>(g, phi, epad, t);
 }
 
 // One n^3 FP64 component array -> that component of every padded E node (uploaded E).
@@ -371,12 +186,13 @@ struct SpeciesCharges {
 // Four nodes per thread per iteration, every weight-sum load of the four issued
 // before the first node is formed: one node at a time, the kernel waited on two
 // dependent-free loads per node and ran at a third of its bytes' bandwidth.
-__global__ void k_wsum_to_rho(const unsigned long long *w, int64_t ncell, SpeciesCharges sc, float *rho)
+// The charges' integer form comes from the host (computing it in each block was
+// most of the kernel on a small grid), and the sums are cleared for the next
+// deposit as they are read, which saves that deposit's clear.
+__global__ void k_wsum_to_rho(unsigned long long *w, int64_t ncell, const __grid_constant__ SpeciesCharges sc,
+                              const __grid_constant__ RhoScale r, float *rho)
 {
     constexpr int U = 4;
-    __shared__ RhoScale r;
-    if (threadIdx.x == 0) r = rho_scale(sc.q, sc.nspecies);
-    __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ncell; t += U * stride) {
         unsigned long long W[U][2];
@@ -393,18 +209,28 @@ __global__ void k_wsum_to_rho(const unsigned long long *w, int64_t ncell, Specie
             if (!in[u]) continue;
             const int64_t i = t + u * stride;
             rho[i] = sc.nspecies <= 2 ? node_rho2(W[u], sc.nspecies, sc.q, r) : node_rho(w + i, ncell, sc.nspecies, sc.q, r);
+            for (int s = 0; s < sc.nspecies; ++s) w[s * ncell + i] = 0ull;
         }
     }
 }
 
 // FP64 form: rho = (sum_s q_s W_s) 2^-48 from the species' 2^-48 fixed-point
 // weight sums, the species added in a fixed order, so rho is bit-reproducible.
-__global__ void k_wsum_to_rho64(const unsigned long long *w, int64_t ncell, SpeciesCharges sc, double *rho)
+__global__ void k_wsum_to_rho64(unsigned long long *w, int64_t ncell, SpeciesCharges sc, double *rho)
 {
     constexpr double kUnit48 = 1.0 / 281474976710656.0;   // 2^-48
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ncell; t += (int64_t)gridDim.x * blockDim.x) {
+        unsigned long long W[OHPIC_MAX_SPECIES];
+#pragma unroll
+        for (int s = 0; s < OHPIC_MAX_SPECIES; ++s)
+            if (s < sc.nspecies) W[s] = w[s * ncell + t];
         double acc = 0.0;
-        for (int s = 0; s < sc.nspecies; ++s) acc += sc.q[s] * (double)w[s * ncell + t];
+#pragma unroll
+        for (int s = 0; s < OHPIC_MAX_SPECIES; ++s)
+            if (s < sc.nspecies) {
+                acc += sc.q[s] * (double)W[s];
+                w[s * ncell + t] = 0ull;
+            }
         rho[t] = acc * kUnit48;
     }
 }
@@ -418,7 +244,8 @@ int blocks_for(int64_t n)
 
 }  // namespace
 
-// Materialise rho from the fixed-point weight sums left by the last deposit.
+// Materialise rho from the fixed-point weight sums left by the last deposit, and
+// clear them.
 void ensure_rho(ohpic_ctx *c)
 {
     if (!c->rho_from_wsum) return;
@@ -426,11 +253,13 @@ void ensure_rho(ohpic_ctx *c)
     sc.nspecies = c->cfg.nspecies;
     for (int s = 0; s < OHPIC_MAX_SPECIES; ++s) sc.q[s] = s < sc.nspecies ? c->cfg.q[s] : 0.0;
     if (c->cfg.precision == OHPIC_FP32)
-        k_wsum_to_rho<<<blocks_for(c->g.ncell), 256, 0, c->stream>>>(c->wsum, c->g.ncell, sc, (float *)c->rho);
+        k_wsum_to_rho<<<blocks_for(c->g.ncell), 256, 0, c->stream>>>(c->wsum, c->g.ncell, sc,
+                                                                     rho_scale(sc.q, sc.nspecies), (float *)c->rho);
     else
         k_wsum_to_rho64<<<blocks_for(c->g.ncell), 256, 0, c->stream>>>(c->wsum, c->g.ncell, sc, (double *)c->rho);
     ++c->launches;
     c->rho_from_wsum = false;
+    c->wsum_clear = true;
 }
 
 int fields_setup(ohpic_ctx *c)
@@ -465,7 +294,7 @@ void fields_teardown(ohpic_ctx *c)
     }
 }
 
-int solve_fields(ohpic_ctx *c)
+int solve_fields(ohpic_ctx *c, unsigned long long *clear, int nclear)
 {
     const Geom &g = c->g;
     ensure_rho(c);
@@ -476,16 +305,16 @@ int solve_fields(ohpic_ctx *c)
         k_scale_z<<<blocks_for(g.nspec), 256, 0, c->stream>>>((cufftDoubleComplex *)c->spec, c->green, g.nspec);
         r = cufftExecZ2D(c->plan_c2r, (cufftDoubleComplex *)c->spec, (cufftDoubleReal *)c->phi);
         if (r != CUFFT_SUCCESS) goto fail;
-        k_stencil<double, dnode><<<blocks_for((int64_t)g.gx * g.gy * g.gz), 256, 0, c->stream>>>(
-            g, (const double *)c->phi, (dnode *)c->epad);
+        launch_stencil<double, dnode>(c->stream, g, 1, (const double *)c->phi, (dnode *)c->epad, nullptr, clear,
+                                      nclear);
     } else {
         r = cufftExecR2C(c->plan_r2c, (cufftReal *)c->rho, (cufftComplex *)c->spec);
         if (r != CUFFT_SUCCESS) goto fail;
         k_scale_c<<<blocks_for(g.nspec), 256, 0, c->stream>>>((cufftComplex *)c->spec, c->green, g.nspec);
         r = cufftExecC2R(c->plan_c2r, (cufftComplex *)c->spec, (cufftReal *)c->phi);
         if (r != CUFFT_SUCCESS) goto fail;
-        k_stencil<float, float4><<<blocks_for((int64_t)g.gx * g.gy * g.gz), 256, 0, c->stream>>>(
-            g, (const float *)c->phi, (float4 *)c->epad);
+        launch_stencil<float, float4>(c->stream, g, 1, (const float *)c->phi, (float4 *)c->epad, nullptr, clear,
+                                      nclear);
     }
     c->launches += 2;
     return OHPIC_OK;
@@ -507,6 +336,7 @@ int pool_green(cudaStream_t st, const Geom &g, double *green)
 int pool_solve(cudaStream_t st, const FieldPool &p)
 {
     const Geom &g = p.g;
+    if (p.spectral) return spectral_solve(*p.spectral, st, p) == cudaSuccess ? 4 : -1;
     const unsigned slots = (unsigned)p.slots;
     auto grid = [&](int64_t n) {
         int64_t b = (n + 255) / 256;
@@ -518,7 +348,7 @@ int pool_solve(cudaStream_t st, const FieldPool &p)
     if (cufftExecR2C(p.r2c, p.rho, p.spec) != CUFFT_SUCCESS) return -1;
     k_pool_scale<<<grid(g.nspec), 256, 0, st>>>(p.spec, g.nspec, p.green, p.on);
     if (cufftExecC2R(p.c2r, p.spec, p.phi) != CUFFT_SUCCESS) return -1;
-    k_pool_stencil<<<grid((int64_t)g.gx * g.gy * g.gz), 256, 0, st>>>(g, p.phi, p.epad, p.on);
+    launch_stencil<float, float4>(st, g, p.slots, p.phi, p.epad, p.on, nullptr, 0);
     return 5;
 }
 

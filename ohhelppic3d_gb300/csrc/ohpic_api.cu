@@ -217,7 +217,8 @@ int check_upload(ohpic_ctx *c, int s)
 // solve or download.
 void zero_deposit(ohpic_ctx *c)
 {
-    launch_zero(c, c->wsum, (int64_t)c->cfg.nspecies * c->g.ncell * 8);
+    if (!c->wsum_clear) launch_zero(c, c->wsum, (int64_t)c->cfg.nspecies * c->g.ncell * 8);
+    c->wsum_clear = false;
     c->rho_from_wsum = true;
 }
 
@@ -229,19 +230,28 @@ int do_scatter(ohpic_ctx *c)
     return OHPIC_OK;
 }
 
-int do_solve(ohpic_ctx *c)
+// The push's tallies (crossings, particles outside their tile, and the kinetic
+// sums when it tracks them): the leading bytes of DevDiag.
+size_t tally_bytes(const ohpic_ctx *c) { return c->with_energy ? offsetof(DevDiag, charge) : offsetof(DevDiag, kin); }
+
+// push_next: a push follows at once, so the solve's last kernel clears its tallies.
+int do_solve(ohpic_ctx *c, bool push_next = false)
 {
     if (!c->rho_valid) do_scatter(c);
-    const int rc = solve_fields(c);
-    if (rc == OHPIC_OK) c->field_valid = true;
+    const int rc = push_next ? solve_fields(c, (unsigned long long *)c->diag, (int)(tally_bytes(c) / 8))
+                             : solve_fields(c, nullptr, 0);
+    if (rc == OHPIC_OK) {
+        c->field_valid = true;
+        c->diag_clear = push_next;
+    }
     return rc;
 }
 
 int do_push(ohpic_ctx *c, double dt)
 {
     set_dt(c, dt);
-    // crossings + outside (+ the kinetic sums when the push tracks them)
-    cudaMemsetAsync(c->diag, 0, c->with_energy ? offsetof(DevDiag, charge) : offsetof(DevDiag, kin), c->stream);
+    if (!c->diag_clear) cudaMemsetAsync(c->diag, 0, tally_bytes(c), c->stream);
+    c->diag_clear = false;
     c->kin_valid = c->with_energy;
     zero_deposit(c);
     if (c->push_timing) {
@@ -723,7 +733,7 @@ int ohpic_push(ohpic_ctx *c, double dt)
     if (!c || !std::isfinite(dt)) return fail(c, OHPIC_ERR_INVALID, "push: bad dt");
     cudaSetDevice(c->dev);
     if (!c->field_valid) {
-        const int rc = do_solve(c);
+        const int rc = do_solve(c, true);
         if (rc != OHPIC_OK) return rc;
     }
     return do_push(c, dt);
@@ -745,7 +755,7 @@ int ohpic_step(ohpic_ctx *c, double dt, int nsteps)
         if (rc != OHPIC_OK) return rc;
     }
     for (int i = 0; i < nsteps; ++i) {
-        int rc = do_solve(c);
+        int rc = do_solve(c, true);
         if (rc == OHPIC_OK) rc = do_push(c, dt);
         if (rc == OHPIC_OK && c->cfg.sort_every > 0 && c->steps_since_sort >= c->cfg.sort_every)
             rc = sort_particles(c);

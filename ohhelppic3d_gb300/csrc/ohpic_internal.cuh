@@ -179,6 +179,8 @@ struct MultiSort {
     uint32_t *cursor;           // zeroed before the scatter
 };
 
+struct Spectral;
+
 // Fields of many runs of one grid size (serve.cu): slot k owns the k-th n^3 block
 // of rho and phi, the k-th spectrum and padded E, and nsp weight-sum arrays;
 // one batched cuFFT plan pair covers every slot.
@@ -193,6 +195,7 @@ struct FieldPool {
     double *green;                  // shared by the slots (same grid)
     double *q;                      // [slot][nsp] species charges
     int *on;                        // [slot] 1 when a run owns the slot
+    struct Spectral *spectral;      // our own transforms (spectral.cu); null: the cuFFT plans
     cufftHandle r2c, c2r;
 };
 
@@ -230,6 +233,8 @@ struct ohpic_ctx {
     // depend on the order of the atomics); the solve turns them into rho.
     unsigned long long *wsum;
     bool rho_from_wsum;
+    bool wsum_clear;        // the weight sums are zero (cleared by the kernel that read them)
+    bool diag_clear;        // the push's tallies are zero (cleared by the solve just before it)
     // TMA description of epad for staging a tile's E box (tma_map.cu).
     CUtensorMap emap;   // carries its own alignment
     bool emap_ok;
@@ -308,7 +313,16 @@ void ensure_emap(ohpic_ctx *c);
 // Fields (fields.cu).
 int fields_setup(ohpic_ctx *c);
 void fields_teardown(ohpic_ctx *c);
-int solve_fields(ohpic_ctx *c);
+// clear, when given: nclear 8-byte words the solve's last kernel zeroes.
+int solve_fields(ohpic_ctx *c, unsigned long long *clear, int nclear);
+// The pooled field solve with our own transforms (spectral.cu): null when the
+// grid's planes or prime factors are too large for it (and on a failed allocation).
+Spectral *spectral_create(const Geom &g, const double *green);
+void spectral_destroy(Spectral *s);
+cudaError_t spectral_solve(const Spectral &s, cudaStream_t st, const FieldPool &p);
+template <typename T, typename NodeT>
+void launch_stencil(cudaStream_t st, const Geom &g, int slots, const T *phi, NodeT *epad, const int *on,
+                    unsigned long long *clear, int nclear);
 void launch_zero(ohpic_ctx *c, void *p, int64_t bytes);
 int pool_green(cudaStream_t st, const Geom &g, double *green);
 int pool_solve(cudaStream_t st, const FieldPool &p);

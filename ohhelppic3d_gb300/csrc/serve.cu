@@ -372,6 +372,9 @@ Pool *create_pool(Server *s, const Geom &g, std::string &why)
         cudaMemsetAsync(f.q, 0, (size_t)slots * nsp * 8, s->st);
         cudaMemsetAsync(f.on, 0, (size_t)slots * 4, s->st);
         pool_green(s->st, g, f.green);
+        f.spectral = spectral_create(g, f.green);
+    }
+    if (ok && !f.spectral) {
         int dims[3] = {g.nz, g.ny, g.nx};
         ok = cufftPlanMany(&f.r2c, 3, dims, nullptr, 1, (int)g.ncell, nullptr, 1, (int)g.nspec, CUFFT_R2C, slots) ==
              CUFFT_SUCCESS;
@@ -387,18 +390,21 @@ Pool *create_pool(Server *s, const Geom &g, std::string &why)
         } else {
             why = "cufftPlanMany failed";
         }
-    } else {
+    } else if (!ok) {
         why = "pool allocation failed";
     }
     if (!ok) {
+        spectral_destroy(f.spectral);
         for (void *p : {(void *)f.rho, (void *)f.phi, (void *)f.spec, (void *)f.epad, (void *)f.wsum, (void *)f.green,
                         (void *)f.q, (void *)f.on})
             sfree(s, p);
         return nullptr;
     }
     size_t w1 = 0, w2 = 0;
-    cufftGetSize(f.r2c, &w1);
-    cufftGetSize(f.c2r, &w2);
+    if (P->plans) {
+        cufftGetSize(f.r2c, &w1);
+        cufftGetSize(f.c2r, &w2);
+    }
     P->bytes = pool_bytes(g, slots, nsp) + (int64_t)(w1 + w2);
     P->owner.assign(slots, -1);
     P->q.assign((size_t)slots * nsp, 0.0);
@@ -419,6 +425,8 @@ void destroy_pool(Server *s, Pool *P)
         cufftDestroy(f.c2r);
         P->plans = false;
     }
+    spectral_destroy(f.spectral);
+    f.spectral = nullptr;
     for (void *p : {(void *)f.rho, (void *)f.phi, (void *)f.spec, (void *)f.epad, (void *)f.wsum, (void *)f.green,
                     (void *)f.q, (void *)f.on})
         sfree(s, p);
