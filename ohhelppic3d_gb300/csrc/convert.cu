@@ -2,6 +2,7 @@
 // device forms, kinetic-energy reduction, and the dispatch of the tiled kernels.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include "ohpic_internal.cuh"
 
@@ -247,9 +248,10 @@ int pick_split(const ohpic_ctx *c)
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-void launch_tiled(ohpic_ctx *c, int mode, int strict)
+TileArgs tile_args(ohpic_ctx *c, int mode)
 {
     TileArgs a;
+    memset(&a, 0, sizeof(a));   // compared as bytes
     a.g = c->g;
     a.nspecies = c->cfg.nspecies;
     a.weights = c->cfg.weights;
@@ -273,7 +275,12 @@ void launch_tiled(ohpic_ctx *c, int mode, int strict)
     a.wsum = c->wsum;
     a.interp_out = c->interp_buf;
     a.diag = c->diag;
+    return a;
+}
 
+void launch_tiled(ohpic_ctx *c, int mode, int strict)
+{
+    const TileArgs a = tile_args(c, mode);
     const bool f64 = c->cfg.precision == OHPIC_FP64;
     // particles per thread per iteration: 2 in both forms (double2 / float2 vectors)
     const int PPT = 2;

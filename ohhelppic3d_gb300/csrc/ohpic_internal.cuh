@@ -281,6 +281,14 @@ struct ohpic_ctx {
     bool with_energy;
     bool kin_valid;             // diag->kin holds the sums of the current velocities
 
+    // A captured step (solve and push) and what it was captured for (ohpic_api.cu).
+    cudaGraphExec_t step_graph;
+    ohpic::TileArgs step_args;
+    int step_flags;
+    int64_t step_launches;
+    bool step_graph_off;        // capture failed once: plain launches from then on
+    bool step_launched;         // a step has been launched plainly (its kernels are loaded)
+
     int64_t launches;
     int64_t push_launches;
     bool push_timing;
@@ -300,6 +308,8 @@ void species_consts(const ohpic_config &cfg, int s, double dt, SpeciesConst &k);
 
 // Kernel launchers: dispatch (convert.cu) and the two forms (push_f64.cu, push_f32.cu).
 void launch_tiled(ohpic_ctx *c, int mode, int strict);
+// The arguments of the tiled kernels for the context's current state.
+TileArgs tile_args(ohpic_ctx *c, int mode);
 void launch_tiled_f64(ohpic_ctx *c, const TileArgs &a, int mode, int strict, int64_t blocks, size_t smem);
 void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks, size_t smem,
                       const RecIn *rin = nullptr);
