@@ -17,6 +17,7 @@
 #include <cufft.h>
 #include <stdint.h>
 
+#include "block_sum.cuh"
 #include "field_nodes.cuh"
 #include "ohpic_internal.cuh"
 
@@ -158,22 +159,17 @@ template <typename T, typename NodeT>
 __global__ void k_field_sums(Geom g, const T *rho, const NodeT *epad, double *charge, double *energy)
 {
     double q = 0.0, e2 = 0.0;
+    // at most 2^31 cells: the node comes from 32-bit divisions
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < g.ncell; t += (int64_t)gridDim.x * blockDim.x) {
         q += (double)rho[t];
-        const int i = (int)(t % g.nx);
-        const int j = (int)((t / g.nx) % g.ny);
-        const int k = (int)(t / ((int64_t)g.nx * g.ny));
+        const unsigned row = (unsigned)t / (unsigned)g.nx, k = row / (unsigned)g.ny;
+        const int i = (int)((unsigned)t - row * (unsigned)g.nx), j = (int)(row - k * (unsigned)g.ny);
         const NodeT e = epad[(i + g.halo) + (int64_t)g.gx * ((j + g.halo) + (int64_t)g.gy * (k + g.halo))];
         e2 += (double)e.x * (double)e.x + (double)e.y * (double)e.y + (double)e.z * (double)e.z;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        q += __shfl_xor_sync(0xffffffffu, q, o);
-        e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(charge, q);
-        atomicAdd(energy, 0.5 * e2);
-    }
+    double v[2] = {q, 0.5 * e2};
+    double *const out[2] = {charge, energy};
+    block_sum_add(v, out);
 }
 
 // FP32 form: rho = sum_s q_s * W_s * 2^-24 from the fixed-point weight sums,

@@ -187,13 +187,16 @@ void dfree(void *p)
 // Device error flag raised by a kernel (bounds), read after a synchronise.
 int check_device(ohpic_ctx *c)
 {
-    cudaError_t e = cudaStreamSynchronize(c->stream);
+    // both words ride behind the work into pinned memory: one wait instead of a
+    // wait and two blocking copies
+    cudaError_t e = cudaMemcpyAsync(&c->diag_host->err_code, &c->diag->err_code, 2 * sizeof(int),
+                                    cudaMemcpyDeviceToHost, c->stream);
+    const cudaError_t se = cudaStreamSynchronize(c->stream);
+    if (se != cudaSuccess) e = se;
     if (e != cudaSuccess) return fail(c, OHPIC_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(c, OHPIC_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-    int code = 0, info = 0;
-    cudaMemcpy(&code, &c->diag->err_code, sizeof(int), cudaMemcpyDeviceToHost);
-    cudaMemcpy(&info, &c->diag->err_info, sizeof(int), cudaMemcpyDeviceToHost);
+    const int code = c->diag_host->err_code, info = c->diag_host->err_info;
     if (code != 0) {
         cudaMemset(&c->diag->err_code, 0, 2 * sizeof(int));
         return fail(c, code, "device error flag " + std::to_string(code) + " at site " + std::to_string(info));
@@ -790,7 +793,7 @@ int ohpic_interp(ohpic_ctx *c, int s, double *e_out, int64_t capacity, int64_t *
         c->interp_cap = need;
     }
     const int strict = 1;
-    launch_tiled(c, MODE_INTERP, strict);
+    launch_tiled(c, MODE_INTERP, strict, s);   // the other species' slots are not asked for
     if (n > 0)
         OHPIC_CUDA_TRY(c, cudaMemcpyAsync(e_out, c->interp_buf + 3 * c->seg[s], sizeof(double) * 3 * n,
                                           cudaMemcpyDeviceToHost, c->stream));

@@ -127,7 +127,8 @@ struct TileArgs {
     unsigned long long *wsum;          // [species][n^3] sums of CIC weights, 2^-24 (FP32) or 2^-48 (FP64) fixed point
     double *interp_out;                // MODE_INTERP: 3 per particle slot (absolute index)
     DevDiag *diag;
-    int chunk;                         // particles per CTA when unsorted
+    int chunk;                         // particles per CTA when unsorted (a multiple of 4)
+    int sp0, nsp;                      // the launch covers species [sp0, sp0 + nsp)
 };
 
 // Sorted 32-byte particle records (sort.cu) read by the push that follows the
@@ -307,9 +308,10 @@ bool make_geom(const ohpic_config &k, const int tile[3], int halo, Geom &g, cons
 void species_consts(const ohpic_config &cfg, int s, double dt, SpeciesConst &k);
 
 // Kernel launchers: dispatch (convert.cu) and the two forms (push_f64.cu, push_f32.cu).
-void launch_tiled(ohpic_ctx *c, int mode, int strict);
+// species: the one species to run (MODE_INTERP), or -1 for all.
+void launch_tiled(ohpic_ctx *c, int mode, int strict, int species = -1);
 // The arguments of the tiled kernels for the context's current state.
-TileArgs tile_args(ohpic_ctx *c, int mode);
+TileArgs tile_args(ohpic_ctx *c, int mode, int species = -1);
 void launch_tiled_f64(ohpic_ctx *c, const TileArgs &a, int mode, int strict, int64_t blocks, size_t smem);
 void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks, size_t smem,
                       const RecIn *rin = nullptr);

@@ -52,6 +52,7 @@
 #include <thread>
 #include <vector>
 
+#include "block_sum.cuh"
 #include "ohpic_internal.cuh"
 #include "../../include/ohpic_serve.h"
 
@@ -86,18 +87,9 @@ __global__ void k_run_kinetic(PartF32 p, int64_t seg, int64_t n, double *out4)
         ke += vx * vx + vy * vy + vz * vz;
         mx += vx; my += vy; mz += vz;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        ke += __shfl_xor_sync(0xffffffffu, ke, o);
-        mx += __shfl_xor_sync(0xffffffffu, mx, o);
-        my += __shfl_xor_sync(0xffffffffu, my, o);
-        mz += __shfl_xor_sync(0xffffffffu, mz, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(out4 + 0, ke);
-        atomicAdd(out4 + 1, mx);
-        atomicAdd(out4 + 2, my);
-        atomicAdd(out4 + 3, mz);
-    }
+    double v[4] = {ke, mx, my, mz};
+    double *const out[4] = {out4, out4 + 1, out4 + 2, out4 + 3};
+    block_sum_add(v, out);
 }
 
 // Particles of one species in injection order (ids are the injector's indices):

@@ -124,8 +124,9 @@ __device__ __forceinline__ bool get_item(const TileArgs &a, int64_t b, Item &it)
 {
     if (a.sorted) {
         const int64_t per_sp = a.g.ntile * a.split;
-        it.sp = (int)(b / per_sp);
-        const int64_t r = b % per_sp;
+        const int64_t s = b / per_sp;
+        it.sp = a.sp0 + (int)s;
+        const int64_t r = b - s * per_sp;
         it.tile = (int)(r / a.split);
         const int part = (int)(r % a.split);
         const int64_t *tb = a.tile_begin + (int64_t)it.sp * (a.g.ntile + 1);
@@ -141,15 +142,15 @@ __device__ __forceinline__ bool get_item(const TileArgs &a, int64_t b, Item &it)
         it.z0 = tz * a.g.tz;
     } else {
         // Unsorted: consecutive chunks of every species, no staging.
-        int sp = 0;
+        int sp = a.sp0;
         int64_t first = 0;
-        for (; sp < a.nspecies; ++sp) {
+        for (; sp < a.sp0 + a.nsp; ++sp) {
             const int64_t groups = (a.count[sp] + PPT - 1) / PPT;
             const int64_t blocks = (groups * PPT + a.chunk - 1) / a.chunk;
             if (b < first + blocks) break;
             first += blocks;
         }
-        if (sp >= a.nspecies) return false;
+        if (sp >= a.sp0 + a.nsp) return false;
         it.sp = sp;
         it.tile = -1;
         const int64_t gseg = a.seg[sp] / PPT;
