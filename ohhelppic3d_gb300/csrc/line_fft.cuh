@@ -6,8 +6,9 @@
 // multiplies element i by exp(-2 pi i k i / (L R)), transforms the R of them and
 // writes them at (p - k) R + k + i L.  Consecutive threads take consecutive
 // lines, so a line's butterflies share their twiddles (a broadcast) and shared
-// accesses run across lines.  Radices 2, 3, 4, 5, 7 and 8 keep a butterfly in
-// registers; a larger prime up to kMaxPrime takes one thread per output.
+// accesses run across lines.  Radices 2 to 5, 7, 8, 11 and 13 keep a
+// butterfly in registers; a larger prime takes one thread per
+// output or two.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -19,7 +20,6 @@
 namespace ohpic {
 namespace {
 
-constexpr int kMaxPrime = 31;
 constexpr int kMaxStages = 10;
 
 // x / d for 0 <= x, d < 2^16 with one high multiply.
@@ -39,8 +39,9 @@ struct LinePlan {
     FastDiv L[kMaxStages];
 };
 
-// False when n has a prime factor above kMaxPrime or does not fit the index arithmetic.
-inline bool line_plan(int n, LinePlan &p)
+// False when n has a prime factor above max_prime (at most 67) or does not fit the
+// index arithmetic.
+inline bool line_plan(int n, LinePlan &p, int max_prime = 31)
 {
     p.n = n;
     p.nst = 0;
@@ -53,6 +54,11 @@ inline bool line_plan(int n, LinePlan &p)
         L *= r;
         left /= r;
     };
+    for (int q : {67, 61, 59, 53, 47, 43, 41, 37, 31, 29, 23, 19, 17})
+        if (q <= max_prime && left % q == 0) {   // a large prime first, where it has no twiddles
+            take(q);
+            break;
+        }
     while (left > 1) {
         if (p.nst == kMaxStages) return false;
         int r = 0;
@@ -60,8 +66,8 @@ inline bool line_plan(int n, LinePlan &p)
         else if (left % 8 == 0) r = 8;
         else if (left % 4 == 0) r = 4;
         else
-            for (int q : {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31})
-                if (left % q == 0) {
+            for (int q : {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67})
+                if (q <= max_prime && left % q == 0) {
                     r = q;
                     break;
                 }
@@ -152,22 +158,46 @@ __device__ __forceinline__ void dft4(V &a, V &b, V &c, V &d)
 template <int R>
 __device__ __forceinline__ constexpr double odd_cos(int q)
 {
-    if (R == 3) return q == 0 ? 1.0 : -0.5;
-    if (R == 5) return q == 0 ? 1.0 : q == 1 ? 0.30901699437494742410 : -0.80901699437494742410;
-    return q == 0   ? 1.0
-           : q == 1 ? 0.62348980185873353053
-           : q == 2 ? -0.22252093395631440429
-                    : -0.90096886790241912624;
+    if (R == 3)
+        return q == 0 ? 1.0 : -0.500000000000000000000;
+    if (R == 5)
+        return q == 0 ? 1.0 : q == 1 ? 0.309016994374947424102 : 
+               -0.809016994374947424102;
+    if (R == 7)
+        return q == 0 ? 1.0 : q == 1 ? 0.623489801858733530525 : 
+               q == 2 ? -0.222520933956314404289 : -0.900968867902419126236;
+    if (R == 11)
+        return q == 0 ? 1.0 : q == 1 ? 0.841253532831181168862 : 
+               q == 2 ? 0.415415013001886425529 : q == 3 ? -0.142314838273285140444 : 
+               q == 4 ? -0.654860733945285064057 : -0.959492973614497389890;
+    if (R == 13)
+        return q == 0 ? 1.0 : q == 1 ? 0.885456025653209895900 : 
+               q == 2 ? 0.568064746731155802512 : q == 3 ? 0.120536680255323053349 : 
+               q == 4 ? -0.354604887042535625970 : q == 5 ? -0.748510748171101098635 : 
+               -0.970941817426052027157;
+    return 0.0;
 }
 template <int R>
 __device__ __forceinline__ constexpr double odd_sin(int q)
 {
-    if (R == 3) return q == 0 ? 0.0 : 0.86602540378443864676;
-    if (R == 5) return q == 0 ? 0.0 : q == 1 ? 0.95105651629515357212 : 0.58778525229247312917;
-    return q == 0   ? 0.0
-           : q == 1 ? 0.78183148246802980871
-           : q == 2 ? 0.97492791218182360702
-                    : 0.43388373911755812048;
+    if (R == 3)
+        return q == 0 ? 0.0 : 0.866025403784438646764;
+    if (R == 5)
+        return q == 0 ? 0.0 : q == 1 ? 0.951056516295153572116 : 
+               0.587785252292473129169;
+    if (R == 7)
+        return q == 0 ? 0.0 : q == 1 ? 0.781831482468029808708 : 
+               q == 2 ? 0.974927912181823607018 : 0.433883739117558120476;
+    if (R == 11)
+        return q == 0 ? 0.0 : q == 1 ? 0.540640817455597582108 : 
+               q == 2 ? 0.909631995354518371412 : q == 3 ? 0.989821441880932732376 : 
+               q == 4 ? 0.755749574354258283774 : 0.281732556841429697711;
+    if (R == 13)
+        return q == 0 ? 0.0 : q == 1 ? 0.464723172043768545656 : 
+               q == 2 ? 0.822983865893656394580 : q == 3 ? 0.992708874098053992801 : 
+               q == 4 ? 0.935016242685414823440 : q == 5 ? 0.663122658240795202377 : 
+               0.239315664287557767149;
+    return 0.0;
 }
 
 // Odd R from the sums and differences of the elements k and R - k.
@@ -240,12 +270,13 @@ __device__ __forceinline__ void dft(V v[R])
     }
 }
 
-// One stage over every line: element e of line l sits at l * ls + e * es.
+// One stage over every line: element e of line l sits at l * ls + e * es.  tw is a
+// table of n * ts roots, so exp(-2 pi i k / n) is its entry k * ts.
 template <int R, typename V>
 __device__ __forceinline__ void line_stage(const V *in, V *out, unsigned lines, FastDiv dl, int n, int es, int ls,
-                                           FastDiv dL, const V *tw)
+                                           FastDiv dL, const V *tw, int ts)
 {
-    const int L = (int)dL.d, m = n / R, step = n / (L * R);
+    const int L = (int)dL.d, m = n / R, step = n / (L * R) * ts;
     for (unsigned t = threadIdx.x; t < lines * (unsigned)m; t += blockDim.x) {
         const int p = (int)div_by(dl, t), line = (int)t - p * (int)lines;
         const int q = (int)div_by(dL, (unsigned)p), k = p - q * L;
@@ -267,7 +298,7 @@ __device__ __forceinline__ void line_stage(const V *in, V *out, unsigned lines, 
 // A larger prime radix: one thread per output, a running twiddle index.
 template <typename V>
 __device__ __forceinline__ void line_stage_prime(int R, const V *in, V *out, unsigned lines, FastDiv dl, int n, int es,
-                                                 int ls, FastDiv dL, const V *tw)
+                                                 int ls, FastDiv dL, const V *tw, int ts)
 {
     const int L = (int)dL.d, m = n / R, step = n / (L * R);
     for (unsigned t = threadIdx.x; t < lines * (unsigned)n; t += blockDim.x) {
@@ -281,9 +312,62 @@ __device__ __forceinline__ void line_stage_prime(int R, const V *in, V *out, uns
         for (int s = 1; s < R; ++s) {
             w += inc;
             if (w >= n) w -= n;
-            acc = cadd(acc, cmul(src[s * m * es], tw[w]));
+            acc = cadd(acc, cmul(src[s * m * es], tw[w * ts]));
         }
         out[line * ls + (q * L * R + k + i * L) * es] = acc;
+    }
+}
+
+// A larger prime radix as the first stage (no twiddles): one thread per outputs i and
+// R - i, from the sums and differences of the elements s and R - s.
+template <typename V>
+__device__ __forceinline__ void line_first_prime(int R, const V *in, V *out, unsigned lines, FastDiv dl, int n, int es,
+                                                 int ls, const V *tw, int ts)
+{
+    const int m = n / R, H = (R - 1) / 2;
+    for (unsigned t = threadIdx.x; t < lines * (unsigned)(m * (H + 1)); t += blockDim.x) {
+        const int o = (int)div_by(dl, t), line = (int)t - o * (int)lines;
+        const int i = o / m, p = o - i * m;
+        const V *src = in + line * ls + p * es;
+        V e = src[0], d;
+        d.x = d.y = 0;
+        int w = 0;
+        for (int s = 1; s <= H; ++s) {
+            w += i;
+            if (w >= R) w -= R;
+            const V c = tw[w * m * ts], a = src[s * m * es], b = src[(R - s) * m * es];
+            e.x += c.x * (a.x + b.x);
+            e.y += c.x * (a.y + b.y);
+            d.x -= c.y * (a.x - b.x);      // c.y = -sin
+            d.y -= c.y * (a.y - b.y);
+        }
+        V *dst = out + line * ls + p * R * es;
+        const V q = cmuli(d);
+        dst[i * es] = cadd(e, q);
+        if (i) dst[(R - i) * es] = csub(e, q);
+    }
+}
+
+// Stage s of a plan from in to out (the caller synchronises).
+template <typename V>
+__device__ __forceinline__ void line_fft_stage(const LinePlan &pl, int s, const V *in, V *out, unsigned lines,
+                                               FastDiv dl, int es, int ls, const V *tw, int ts)
+{
+    const int R = pl.r[s];
+    const FastDiv dL = pl.L[s];
+    switch (R) {
+    case 2: line_stage<2>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 3: line_stage<3>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 4: line_stage<4>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 5: line_stage<5>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 7: line_stage<7>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 11: line_stage<11>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 13: line_stage<13>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    case 8: line_stage<8>(in, out, lines, dl, pl.n, es, ls, dL, tw, ts); break;
+    default:
+        if (s == 0) line_first_prime(R, in, out, lines, dl, pl.n, es, ls, tw, ts);
+        else line_stage_prime(R, in, out, lines, dl, pl.n, es, ls, dL, tw, ts);
+        break;
     }
 }
 
@@ -295,17 +379,7 @@ __device__ __forceinline__ V *line_fft(const LinePlan &pl, V *a, V *b, unsigned 
                                        const V *tw)
 {
     for (int s = 0; s < pl.nst; ++s) {
-        const int R = pl.r[s];
-        const FastDiv dL = pl.L[s];
-        switch (R) {
-        case 2: line_stage<2>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        case 3: line_stage<3>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        case 4: line_stage<4>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        case 5: line_stage<5>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        case 7: line_stage<7>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        case 8: line_stage<8>(a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        default: line_stage_prime(R, a, b, lines, dl, pl.n, es, ls, dL, tw); break;
-        }
+        line_fft_stage(pl, s, a, b, lines, dl, es, ls, tw, 1);
         __syncthreads();
         V *t = a;
         a = b;

@@ -9,9 +9,16 @@
 //
 // The reference runs FFTW's real-to-real transforms per axis: R2HC/HC2R on a
 // periodic axis, DST-I on a Dirichlet one, DCT-I on a Neumann one, and DST-III /
-// DST-II or DCT-III / DCT-II on the two mixed kinds.  cuFFT has no real-to-real
-// transforms, so each one is a complex DFT of a symmetric extension of the line,
-// with the extension and the output twiddles done by our own kernels:
+// DST-II or DCT-III / DCT-II on the two mixed kinds.
+//
+// Blocks whose lines fit a CTA's shared memory (up to about 600 points, no prime
+// factor above 67) take one kernel per axis and direction (k_line_pass, line_r2r.cuh).
+// Whole solves against the path below (us): 256^3 walls 4058 (9111), 128x96x64 mixed
+// 244 (763), 60x45x33 mixed 88 (208), 33^3 walls 90 (158).
+//
+// The others go through cuFFT.  It has no real-to-real transforms, so each one is a
+// complex DFT of a symmetric extension of the line, with the extension and the
+// output twiddles done by our own kernels:
 //   DCT-I  (L points):  DFT of length 2(L-1) of the even extension,  Y_k = Z_k
 //   DST-I  (L points):  DFT of length 2(L+1) of the odd extension,   Y_k = i Z_{k+1}
 //   DCT-II:             DFT of length 2L of x_0..x_{L-1}, x_{L-1}..x_0,  Y_k = e^{-i pi k/2L} Z_k
@@ -45,16 +52,17 @@
 #include <cmath>
 #include <new>
 #include <string>
+#include <vector>
 
+#include "line_r2r.cuh"
 #include "ohpic_internal.cuh"
+#include "pdl.cuh"
 
 namespace ohpic {
 namespace {
 
 // The reference's pi literal (src/utils/science_constants.f90:4) for the tables.
 constexpr double kRefPi = 3.14159265358979;
-
-enum Xform { XF_R2HC, XF_HC2R, XF_DCT1, XF_DST1, XF_DCT2, XF_DCT3, XF_DST2, XF_DST3 };
 
 struct Axis {
     int kind;        // OHPIC_BC_*
@@ -437,6 +445,285 @@ __global__ void k_efield(Block b, const double *phi, double *e)
     }
 }
 
+// ---------------------------------------------------------------------------
+// The transforms of one axis in one kernel: lines whose buffers fit a CTA's shared
+// memory (line_r2r.cuh).  A solve is then x forward (reading rho and the wall
+// terms), y forward, z forward with the division and z backward, y backward, x
+// backward (writing phi on every node), E: six kernels instead of 22, with one
+// read and one write of the block each.
+// ---------------------------------------------------------------------------
+struct Pass {
+    AxisXf ax;
+    int axis;
+    int fwd, bwd;              // Xform or -1
+    bool from_rho, to_phi;
+    int L0, L1, L2;
+    int64_t lines;             // real lines of the axis
+    int P, Pshift;             // pairs of lines per CTA
+    int nb;                    // CTAs with lines; the rest fill the wall rows of phi
+    bool tw_shared;            // the axis' table is copied to shared memory
+    Block b;
+    const double *inv;         // k_inverse_table
+};
+
+// v plus the wall terms of node g (poisson_solver3d.f90:156-168).
+__device__ __noinline__ double wall_terms(const Block &b, const int g[3], double v)
+{
+    for (int d = 0; d < 3; ++d) {
+        if (g[d] == b.term_node_lo[d]) v += b.term_lo[d];
+        if (g[d] == b.term_node_hi[d]) v += b.term_hi[d];
+    }
+    return v;
+}
+
+// 1 / (table entry x normalisers) of every element, 0 for a zeroed mode: the solve then
+// multiplies instead of dividing (11 FP64 operations an element).
+__global__ void k_inverse_table(const __grid_constant__ Block b, const double *tx, const double *ty, const double *tz,
+                                double *inv)
+{
+    const int64_t total = (int64_t)b.L[0] * b.L[1] * b.L[2];
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = t / b.L[0];
+        const int i = (int)(t - row * b.L[0]), k = (int)(row / b.L[1]), j = (int)(row - (int64_t)k * b.L[1]);
+        const double den = (tx[i] + ty[j]) + tz[k];
+        inv[t] = den == 0.0 || (b.zero_first && t == 0) ? 0.0 : 1.0 / (den * b.norm);
+    }
+}
+
+// First element and stride of real line q.
+__device__ __forceinline__ void line_at(const Pass &p, int64_t q, int64_t &base, int64_t &stride)
+{
+    if (p.axis == 0) {
+        base = q * p.L0;
+        stride = 1;
+    } else if (p.axis == 1) {
+        const int64_t k = q / p.L0;
+        base = q - k * p.L0 + (int64_t)p.L0 * p.L1 * k;
+        stride = p.L0;
+    } else {
+        base = q;
+        stride = (int64_t)p.L0 * p.L1;
+    }
+}
+
+// Value of a node on a wall (x walls first, then y, then z, as k_unpack), or false.
+__device__ __forceinline__ bool wall_node(const Block &b, const int g[3], double &v)
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if (b.wall_lo[d] && g[d] == 0) {
+            v = b.wall_value_lo[d];
+            return true;
+        }
+        if (b.wall_hi[d] && g[d] == b.n[d]) {
+            v = b.wall_value_hi[d];
+            return true;
+        }
+    }
+    return false;
+}
+
+// The logical row (j, k) of phi (element e at src[e * stride]), its periodic images and
+// its x walls, by one warp.
+__device__ __forceinline__ void put_row(const Block &b, double *phi, const double *src, int stride, int L, int j,
+                                        int k, int lane)
+{
+    const int gy0 = j + b.ls[1], gz0 = k + b.ls[2];
+    const int ny = b.kind[1] == OHPIC_BC_PERIODIC && j == 0 ? 2 : 1, nz = b.kind[2] == OHPIC_BC_PERIODIC && k == 0 ? 2 : 1;
+    for (int a = 0; a < nz; ++a)
+        for (int c = 0; c < ny; ++c) {
+            double *row = phi + block_index(b, 0, c ? b.n[1] : gy0, a ? b.n[2] : gz0);
+            for (int e = lane; e < L; e += 32) row[e + b.ls[0]] = src[e * stride];
+            if (lane == 0) {
+                if (b.kind[0] == OHPIC_BC_PERIODIC) row[b.n[0]] = src[0];
+                if (b.wall_lo[0]) row[0] = b.wall_value_lo[0];
+                if (b.wall_hi[0]) row[b.n[0]] = b.wall_value_hi[0];
+            }
+        }
+}
+
+// One pass over the lines of an axis.  Bound by FP64 arithmetic (a 256-interval DST-I
+// pair: about 8500 operations against 16000 for the FFT of the doubled line; the FP64
+// pipe is 72-76% busy at 256^3), then by the barriers between stages.  256^3, walls:
+// 0.62-0.69 ms a pass (1.22 ms for the two of z), against 1.13 ms of cuFFT alone plus
+// 0.2 ms of extension and extraction.
+__global__ void __launch_bounds__(320, 2) k_line_pass(const __grid_constant__ Pass p, const double *rho, double *R, double *phi)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int S = p.P + 1, L = p.ax.L;
+    double2 *A = (double2 *)smem, *B = A + p.ax.E * S;
+    const double2 *Tw = p.ax.T;
+    if (p.tw_shared) {
+        double2 *own = B + p.ax.E * S;
+        const int nt = 2 * p.ax.n1 + p.ax.n2;
+        for (int i = threadIdx.x; i < nt; i += blockDim.x) own[i] = Tw[i];
+        Tw = own;
+    }
+    pdl_wait();
+    if ((int)blockIdx.x >= p.nb) {
+        // rows of phi on a y or z wall
+        const int B0 = p.b.n[0] + 1, B1 = p.b.n[1] + 1, rows = B1 * (p.b.n[2] + 1);
+        for (int r = blockIdx.x - p.nb; r < rows; r += gridDim.x - p.nb) {
+            int g[3] = {1, r % B1, r / B1};
+            const bool wall = (p.b.wall_lo[1] && g[1] == 0) || (p.b.wall_hi[1] && g[1] == p.b.n[1]) ||
+                              (p.b.wall_lo[2] && g[2] == 0) || (p.b.wall_hi[2] && g[2] == p.b.n[2]);
+            if (!wall) continue;
+            for (int x = threadIdx.x; x < B0; x += blockDim.x) {
+                double v = 0.0;
+                g[0] = x;
+                wall_node(p.b, g, v);
+                phi[(int64_t)r * B0 + x] = v;
+            }
+        }
+        return;
+    }
+    const int64_t q0 = (int64_t)blockIdx.x * 2 * p.P;
+    const int total = 2 * p.P * L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    double *Ad = (double *)A;
+    // real line ql of the CTA is part ql & 1 of complex line ql >> 1
+    if (p.axis == 0) {
+        for (int ql = warp; ql < 2 * p.P; ql += warps) {   // a row per warp
+            const int64_t q = q0 + ql;
+            double *dst = Ad + 2 * (ql >> 1) + (ql & 1);
+            if (q >= p.lines) {
+                for (int e = lane; e < L; e += 32) dst[2 * e * S] = 0.0;
+            } else if (p.from_rho) {
+                const int k = (int)((unsigned)q / (unsigned)p.L1), j = (int)q - k * p.L1;
+                const int gy = j + p.b.ls[1], gz = k + p.b.ls[2];
+                const double *src = rho + block_index(p.b, p.b.ls[0], gy, gz);
+                // (one branch, rarely taken: as selects, the six additions ran for every node)
+                const bool row = gy == p.b.term_node_lo[1] || gy == p.b.term_node_hi[1] ||
+                                 gz == p.b.term_node_lo[2] || gz == p.b.term_node_hi[2];
+                for (int e = lane; e < L; e += 32) {
+                    double v = src[e];
+                    const int g[3] = {e + p.b.ls[0], gy, gz};
+                    if (__builtin_expect(row || g[0] == p.b.term_node_lo[0] || g[0] == p.b.term_node_hi[0], 0))
+                        v = wall_terms(p.b, g, v);
+                    dst[2 * e * S] = v;
+                }
+            } else {
+                for (int e = lane; e < L; e += 32) dst[2 * e * S] = R[q * L + e];
+            }
+        }
+    } else {
+        const int ql = threadIdx.x & (2 * p.P - 1);
+        const int64_t q = q0 + ql;
+        int64_t base, stride;
+        line_at(p, q < p.lines ? q : 0, base, stride);
+        for (int t = threadIdx.x; t < total; t += blockDim.x) {
+            const int e = t >> (p.Pshift + 1);
+            Ad[2 * (e * S + (ql >> 1)) + (ql & 1)] = q < p.lines ? R[base + e * stride] : 0.0;
+        }
+    }
+    __syncthreads();
+    const LineCtx c{A, B, Tw, p.P, p.Pshift};
+    if (p.fwd >= 0) line_r2r(p.ax, p.fwd, c);
+    if (p.axis == 2 && p.bwd >= 0) {
+        // division by the table and the product of the normalisers
+        const int ql = threadIdx.x & (2 * p.P - 1);
+        const int64_t q = q0 + ql, stride = (int64_t)p.L0 * p.L1;
+        if (q < p.lines)
+            for (int t = threadIdx.x; t < total; t += blockDim.x) {
+                const int e = t >> (p.Pshift + 1);
+                Ad[2 * (e * S + (ql >> 1)) + (ql & 1)] *= p.inv[q + e * stride];
+            }
+        __syncthreads();
+    }
+    if (p.bwd >= 0) line_r2r(p.ax, p.bwd, c);
+    if (gridDim.x * blockDim.x <= 152u * 512u) pdl_launch();
+    if (p.axis == 0) {
+        for (int ql = warp; ql < 2 * p.P; ql += warps) {
+            const int64_t q = q0 + ql;
+            if (q >= p.lines) break;
+            const double *src = Ad + 2 * (ql >> 1) + (ql & 1);
+            if (p.to_phi) {
+                const int k = (int)((unsigned)q / (unsigned)p.L1), j = (int)q - k * p.L1;
+                put_row(p.b, phi, src, 2 * S, L, j, k, lane);
+            } else {
+                for (int e = lane; e < L; e += 32) R[q * L + e] = src[2 * e * S];
+            }
+        }
+    } else {
+        const int ql = threadIdx.x & (2 * p.P - 1);
+        const int64_t q = q0 + ql;
+        if (q >= p.lines) return;
+        int64_t base, stride;
+        line_at(p, q, base, stride);
+        for (int t = threadIdx.x; t < total; t += blockDim.x) {
+            const int e = t >> (p.Pshift + 1);
+            R[base + e * stride] = Ad[2 * (e * S + (ql >> 1)) + (ql & 1)];
+        }
+    }
+}
+
+__device__ __noinline__ double half_slow(double x) { return 0.5 * x; }
+
+// x / 2 by the exponent (exact; the FP64 pipe only for zero, subnormals and the like).
+__device__ __forceinline__ double half_of(double x)
+{
+    const long long b = __double_as_longlong(x);
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    return __builtin_expect(e - 2u < 2045u, 1) ? __longlong_as_double(b - (1ll << 52)) : half_slow(x);
+}
+
+// E as k_efield, `planes` planes of one block column per thread.  Of the three FP64
+// additions per component, the upper difference of a node is the lower one of its
+// neighbour: taken from the plane before along z and from the neighbouring lane
+// along x.  Bound by FP64 additions (7 per node instead of 12 operations), then by
+// the writes: 256^3 407 -> 283 us.
+__global__ void __launch_bounds__(256) k_efield_columns(const __grid_constant__ Block b, int planes, const double *phi,
+                                                        double *e)
+{
+    const int B0 = b.n[0] + 1, B1 = b.n[1] + 1, B2 = b.n[2] + 1;
+    const unsigned plane = (unsigned)(B0 * B1), nb = (plane + 255u) / 256u;
+    const unsigned zb = blockIdx.x / nb, t = (blockIdx.x - zb * nb) * 256u + threadIdx.x;
+    const int z0 = (int)zb * planes;
+    const bool in = t < plane;
+    const unsigned tt = in ? t : plane - 1;
+    const int y = (int)(tt / (unsigned)B0), x = (int)(tt - (unsigned)y * (unsigned)B0);
+    const int g[2] = {x, y};
+    // neighbours along x and y: a periodic axis wraps at its ends (node n is the image
+    // of node 0); past a wall of the other kinds there is none
+    int lo[2], hi[2];
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+        lo[d] = g[d] - 1;
+        hi[d] = g[d] + 1;
+        if (g[d] == 0) lo[d] = b.kind[d] == OHPIC_BC_PERIODIC ? b.n[d] - 1 : -1;
+        if (g[d] == b.n[d]) hi[d] = b.kind[d] == OHPIC_BC_PERIODIC ? 1 : -1;
+    }
+    const int64_t total = (int64_t)plane * B2;
+    const bool from_lane = (threadIdx.x & 31) != 0 && x > 0;
+    pdl_wait();
+    const double *col = phi + (int64_t)y * B0 + x;
+    double below = 0.0;    // the lower difference along z of the next plane
+    bool have = false;
+    for (int z = z0; z < min(z0 + planes, B2); ++z) {
+        const double *p = col + (int64_t)z * plane;
+        const double p0 = *p;
+        const double up = hi[0] >= 0 ? p0 - p[hi[0] - x] : 0.0;
+        const double side = __shfl_up_sync(0xffffffffu, up, 1);
+        const double dn = from_lane ? side : lo[0] >= 0 ? p[lo[0] - x] - p0 : 0.0;
+        const double ex = lo[0] < 0 ? up : hi[0] < 0 ? dn : half_of(dn + up);
+        const double yu = hi[1] >= 0 ? p0 - p[(hi[1] - y) * B0] : 0.0, yd = lo[1] >= 0 ? p[(lo[1] - y) * B0] - p0 : 0.0;
+        const double ey = lo[1] < 0 ? yu : hi[1] < 0 ? yd : half_of(yd + yu);
+        int zl = z - 1, zh = z + 1;
+        if (z == 0) zl = b.kind[2] == OHPIC_BC_PERIODIC ? b.n[2] - 1 : -1;
+        if (z == b.n[2]) zh = b.kind[2] == OHPIC_BC_PERIODIC ? 1 : -1;
+        const double zu = zh >= 0 ? p0 - col[(int64_t)zh * plane] : 0.0;
+        const double zd = have ? below : zl >= 0 ? col[(int64_t)zl * plane] - p0 : 0.0;
+        const double ez = zl < 0 ? zu : zh < 0 ? zd : half_of(zd + zu);
+        below = zu;
+        have = true;
+        if (in) {
+            double *o = e + (int64_t)z * plane + t;
+            o[0] = ex;
+            o[total] = ey;
+            o[2 * total] = ez;
+        }
+    }
+}
+
 int grid_of(int64_t n)
 {
     int64_t b = (n + 255) / 256;
@@ -461,6 +748,12 @@ struct ohpic_poisson {
     double *table[3] = {nullptr, nullptr, nullptr};
     double *rho = nullptr, *phi = nullptr, *e = nullptr;   // device staging of the host entry point
     cudaStream_t stream = nullptr;
+    bool passes_ok = false;      // every axis fits a CTA's lines: no plans, no B
+    Pass pass[5];                // x, y forward; z both ways; y, x backward
+    size_t pass_smem[5];
+    int pass_threads[5];
+    double2 *pass_table = nullptr;
+    double *inv = nullptr;
     int64_t nodes = 0;
     std::string err;
 };
@@ -481,9 +774,99 @@ void release(ohpic_poisson *p)
         if (p->planned[d]) cufftDestroy(p->plan[d]);
         if (p->table[d]) cudaFree(p->table[d]);
     }
-    for (void *q : {(void *)p->R, (void *)p->B, (void *)p->rho, (void *)p->phi, (void *)p->e})
+    for (void *q : {(void *)p->R, (void *)p->B, (void *)p->pass_table, (void *)p->inv, (void *)p->rho, (void *)p->phi, (void *)p->e})
         if (q) cudaFree(q);
     if (p->stream) cudaStreamDestroy(p->stream);
+}
+
+// The passes of a block whose lines all fit (R is allocated, the tables are set); false
+// leaves the block to cuFFT.
+bool plan_passes(ohpic_poisson *p)
+{
+    const Block &b = p->blk;
+    const int L[3] = {b.L[0], b.L[1], b.L[2]};
+    const int64_t nl = (int64_t)L[0] * L[1] * L[2];
+    AxisXf ax[3];
+    std::vector<double> t;
+    size_t at[3];
+    for (int d = 0; d < 3; ++d) {
+        at[d] = t.size() / 2;
+        if (!axis_plan(p->ax[d].fwd, L[d], ax[d], t)) return false;
+    }
+    if (nl / std::min(std::min(L[0], L[1]), L[2]) > (int64_t)INT32_MAX) return false;
+    for (int i = 0; i < 5; ++i) {
+        const int d = i < 3 ? i : 4 - i;
+        Pass &q = p->pass[i];
+        q.ax = ax[d];
+        q.axis = d;
+        q.fwd = i < 3 ? p->ax[d].fwd : -1;
+        q.bwd = i >= 2 ? p->ax[d].bwd : -1;
+        q.from_rho = i == 0;
+        q.to_phi = i == 4;
+        q.L0 = L[0]; q.L1 = L[1]; q.L2 = L[2];
+        q.lines = nl / L[d];
+        q.b = b;
+        // Four pairs per CTA (64-byte rows along y and z), eight where that still
+        // leaves two CTAs for every SM and fits a half of it, two where four do not:
+        // every SM has only two FP64 lanes, so small blocks are spread over all
+        // (33^3, walls: 8 pairs 200 us, 4 pairs 124 us, 2 pairs 86 us; 128x96x64: 236,
+        // 239, 280 us).  Eight elements per thread where CTAs abound, else four
+        // (256^3, 4 pairs: 4.52 against 4.61 ms; 100x115x24: 271 against 244 us).
+        auto bytes = [&](int P) {
+            return sizeof(double2) * 2 * (size_t)ax[d].E * (P + 1);
+        };
+        q.P = 8;
+        q.Pshift = 3;
+        while (q.P > 2 && (q.lines / (2 * q.P) < 304 || bytes(q.P) > 60 * 1024 || L[d] * q.P > 320 * kPerThread)) {
+            q.P /= 2;
+            --q.Pshift;
+        }
+        const int64_t ctas = q.lines / (2 * q.P);
+        // the table stays in L1 where CTAs abound and its bytes cost one of them (256^3:
+        // 4.15 against 4.43 ms; 60x45x33 91 against 87 us)
+        q.tw_shared = ctas <= 2048;
+        p->pass_smem[i] = bytes(q.P) + (q.tw_shared ? sizeof(double2) * (size_t)(2 * ax[d].n1 + ax[d].n2) : 0);
+        const int each = ctas > 2048 ? kPerThread : ctas > 608 ? kPerThread / 2 : kPerThread / 4;
+        const int need = (L[d] * q.P + each - 1) / each;
+        p->pass_threads[i] = std::min(std::max(32, (need + 31) / 32 * 32), 320);
+        if (p->pass_smem[i] > 100 * 1024 || L[d] * q.P > 320 * kPerThread || 2 * q.P * L[d] > 32768) return false;
+        q.nb = (int)((q.lines + 2 * q.P - 1) / (2 * q.P));
+    }
+    if (cudaFuncSetAttribute(k_line_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess ||
+        cudaMalloc((void **)&p->pass_table, sizeof(double) * std::max<size_t>(t.size(), 2)) != cudaSuccess ||
+        cudaMemcpy(p->pass_table, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (cudaMalloc((void **)&p->inv, sizeof(double) * nl) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    k_inverse_table<<<grid_of(nl), 256>>>(b, p->table[0], p->table[1], p->table[2], p->inv);
+    if (cudaDeviceSynchronize() != cudaSuccess) return false;
+    for (int i = 0; i < 5; ++i) {
+        p->pass[i].ax.T = p->pass_table + at[p->pass[i].axis];
+        p->pass[i].inv = p->inv;
+    }
+    return true;
+}
+
+void solve_by_passes(ohpic_poisson *p, const double *rho, double *phi, double *e, cudaStream_t st)
+{
+    const Block &b = p->blk;
+    const bool walls = b.wall_lo[1] || b.wall_hi[1] || b.wall_lo[2] || b.wall_hi[2];
+    for (int i = 0; i < 5; ++i) {
+        const int extra = i == 4 && walls ? 64 : 0;
+        launch_overlapped(st, dim3((unsigned)(p->pass[i].nb + extra)), dim3((unsigned)p->pass_threads[i]),
+                          p->pass_smem[i], 1, k_line_pass, p->pass[i], rho, p->R, phi);
+    }
+    if (e) {
+        // eight planes per thread share their z differences where two CTAs per SM remain
+        const int64_t nb = ((int64_t)(b.n[0] + 1) * (b.n[1] + 1) + 255) / 256;
+        const int planes = (int)std::max<int64_t>(1, std::min<int64_t>(8, nb * (b.n[2] + 1) / 304));
+        launch_overlapped(st, dim3((unsigned)(nb * ((b.n[2] + planes) / planes))), dim3(256), 0, 1, k_efield_columns, b,
+                          planes, phi, e);
+    }
 }
 
 // forward or backward transform along one axis of p->R
@@ -610,8 +993,7 @@ int ohpic_poisson_create(const int32_t n[3], const int32_t kinds[3], const doubl
     }
     int rc = OHPIC_OK;
     if (cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking) != cudaSuccess) rc = OHPIC_ERR_CUDA;
-    if (rc == OHPIC_OK && (cudaMalloc((void **)&p->R, sizeof(double) * nl) != cudaSuccess ||
-                           cudaMalloc((void **)&p->B, sizeof(double2) * maxb) != cudaSuccess))
+    if (rc == OHPIC_OK && cudaMalloc((void **)&p->R, sizeof(double) * nl) != cudaSuccess)
         rc = pfail(p, OHPIC_ERR_OOM, "poisson: device buffers");
     for (int d = 0; d < 3 && rc == OHPIC_OK; ++d) {
         // the table per axis: squared wave numbers at the element's global node (as
@@ -632,6 +1014,11 @@ int ohpic_poisson_create(const int32_t n[3], const int32_t kinds[3], const doubl
             rc = pfail(p, OHPIC_ERR_OOM, "poisson: table");
             break;
         }
+    }
+    if (rc == OHPIC_OK) p->passes_ok = plan_passes(p);
+    if (rc == OHPIC_OK && !p->passes_ok && cudaMalloc((void **)&p->B, sizeof(double2) * maxb) != cudaSuccess)
+        rc = pfail(p, OHPIC_ERR_OOM, "poisson: device buffers");
+    for (int d = 0; d < 3 && rc == OHPIC_OK && !p->passes_ok; ++d) {
         const Lines &m = p->lines[d];
         int len = m.M, emb = m.M;
         const cufftResult r = cufftPlanMany(&p->plan[d], 1, &len, &emb, 1, m.M, &emb, 1, m.M, CUFFT_Z2Z, (int)m.lines);
@@ -663,6 +1050,12 @@ int ohpic_poisson_solve_device(ohpic_poisson *p, const double *rho, double *phi,
     if (!p || !rho || !phi) return pfail(p, OHPIC_ERR_INVALID, "poisson: null rho or phi");
     cudaSetDevice(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
+    if (p->passes_ok) {
+        solve_by_passes(p, rho, phi, e, st);
+        const cudaError_t pe = cudaGetLastError();
+        if (pe != cudaSuccess) return pfail(p, OHPIC_ERR_CUDA, std::string("poisson: ") + cudaGetErrorString(pe));
+        return OHPIC_OK;
+    }
     const Block &b = p->blk;
     const int64_t nl = (int64_t)b.L[0] * b.L[1] * b.L[2];
     k_pack<<<grid_of(nl), 256, 0, st>>>(b, rho, p->R);

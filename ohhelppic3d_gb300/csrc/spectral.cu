@@ -25,12 +25,12 @@
 
 #include <algorithm>
 #include <cmath>
-#include <utility>
 #include <vector>
 
 #include "field_nodes.cuh"
 #include "line_fft.cuh"
 #include "ohpic_internal.cuh"
+#include "pdl.cuh"
 
 namespace ohpic {
 namespace {
@@ -56,13 +56,6 @@ struct SpecArgs {
     const double *q;       // charges of every slot, [slot][nsp]
     const int *on;         // slot in use
 };
-
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets the next kernel's CTAs come in while this one finishes.  Called late: CTAs
-// let in early pile up on the SMs that happen to have room and unbalance the
-// chip (a solve of 64^3: 28.2 us with the call at the kernels' start, 20.6 us
-// before their last stores, 32.0 us without it).
-__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ V *stage_twiddles(V *dst, const V *src, int n)
 {
@@ -162,7 +155,7 @@ __global__ void k_plane_forward(const __grid_constant__ SpecArgs a, float *rho, 
     else __syncthreads();
     const int k0 = rank * a.W, own = min(a.W, a.nxh - k0);
     const V *S = line_fft(a.ly, F, R, (unsigned)a.W, a.dW, a.W, 1, twy);
-    launch_next();
+    pdl_launch();
     spec += slot * a.nspec + (int64_t)plane * a.ny * a.nxh;
     for (unsigned t = threadIdx.x; t < (unsigned)(a.ny * a.W); t += blockDim.x) {
         const int y = (int)div_by(a.dW, t), kk = (int)t - y * a.W;
@@ -202,7 +195,7 @@ __global__ void k_pencils(const __grid_constant__ SpecArgs a, V *spec)
     }
     __syncthreads();
     const V *Z = line_fft(a.lz, S, S == A ? B : A, (unsigned)a.C, dC, a.C, 1, tw);
-    launch_next();
+    pdl_launch();
     for (int i = threadIdx.x; i < total; i += blockDim.x) {
         const int z = i >> a.Cshift, c = c0 + (i & (a.C - 1));
         if (c < cols) spec[(int64_t)z * cols + c] = Z[i];   // parts still exchanged
@@ -263,7 +256,7 @@ __global__ void k_plane_inverse(const __grid_constant__ SpecArgs a, const V *spe
     }
     __syncthreads();
     const V *R = line_fft(a.lx, G, U, (unsigned)a.Hc, a.dHc, 1, a.px, twx);
-    launch_next();
+    pdl_launch();
     phi += slot * a.ncell + (int64_t)plane * a.nx * a.ny;
     for (unsigned t = threadIdx.x; t < (unsigned)(a.Hc * a.nx); t += blockDim.x) {
         const int hl = (int)div_by(a.dnx, t), x = (int)t - hl * a.nx;
@@ -318,7 +311,7 @@ __global__ void __launch_bounds__(256) k_stencil_columns(const __grid_constant__
         }
         k = k + 1 == g.nz ? 0 : k + 1;
     }
-    launch_next();
+    pdl_launch();
     epad += (int64_t)slot * g.gz * plane + (int64_t)z0 * plane + t;
 #pragma unroll
     for (int u = 0; u < kStencilZ; ++u) {
@@ -331,27 +324,6 @@ __global__ void __launch_bounds__(256) k_stencil_columns(const __grid_constant__
         e.w = T(0);
         epad[(int64_t)u * plane] = e;
     }
-}
-
-// A launch that may begin while the kernel before it in the stream drains.
-template <typename... P, typename... A>
-cudaError_t launch_overlapped(cudaStream_t st, dim3 grid, dim3 block, size_t smem, int cluster, void (*k)(P...),
-                              A &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)cluster;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 }  // namespace
