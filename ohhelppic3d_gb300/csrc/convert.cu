@@ -215,7 +215,7 @@ int grid_for(int64_t n, int threads)
 // that is nearly empty, or that do not fill the first one, wastes the rest.  The
 // split with the least waves x (cost of one CTA) is taken, a CTA costing a fixed
 // part (its boxes, its first loads) and a part per particle, both measured:
-// FP32 18 us + 3.7 ns, FP64 8 us + 51 ns.  A push of 48^3 x 16 ppc in FP64 (432
+// FP32 18 us + 3.7 ns, FP64 8 us + 32 ns.  A push of 48^3 x 16 ppc in FP64 (432
 // tiles of 8 x 8 x 8) goes from 851 us unsplit to 695 us with two CTAs per tile;
 // 16^3 x 64 ppc from 1445 to 157 us.  A split leaves at least 256 particles to a CTA.
 int pick_split(const ohpic_ctx *c)
@@ -224,7 +224,7 @@ int pick_split(const ohpic_ctx *c)
     int64_t total = 0;
     for (int s = 0; s < c->cfg.nspecies; ++s) total += c->count[s];
     const bool f64 = c->cfg.precision == OHPIC_FP64;
-    const double fixed = f64 ? 8.0 : 18.0, per = (f64 ? 0.051 : 0.0037) * (double)total / (double)items;
+    const double fixed = f64 ? 8.0 : 18.0, per = (f64 ? 0.032 : 0.0037) * (double)total / (double)items;
     constexpr int64_t kSlots = 152 * 2;
     int best = 1;
     double least = 0.0;
@@ -241,7 +241,8 @@ int pick_split(const ohpic_ctx *c)
 
 // Particles per CTA of an unsorted launch: enough CTAs for two waves of the chip
 // where there are that many particles, at least one iteration of 256 threads
-// (two particles per thread, four in the FP32 push and deposit) and at most 4096.
+// (one particle per thread in FP64, two in FP32, four in its push and deposit) and at
+// most 4096.
 // With 4096 throughout, 230400 particles ran on 57 CTAs of 152 SMs: the strict
 // FP64 interpolation took 125 us, the move 186 us, the deposit 73 us (the module loop
 // at 24x20x15 x 16 ppc: 0.99 -> 0.60 ms an iteration, with the interpolation of one
@@ -271,7 +272,9 @@ TileArgs tile_args(ohpic_ctx *c, int mode, int species)
     a.use_tma = c->sorted && c->emap_ok ? 1 : 0;
     a.with_energy = c->with_energy ? 1 : 0;
     a.sorted = c->sorted ? 1 : 0;
-    a.ppl = c->cfg.precision == OHPIC_FP32 && (mode == MODE_PUSH || mode == MODE_DEPOSIT) ? c->lane_particles : 2;
+    a.ppl = c->cfg.precision == OHPIC_FP64                ? 1
+            : mode == MODE_PUSH || mode == MODE_DEPOSIT ? c->lane_particles
+                                                        : 2;
     a.tma_polls = c->tma_polls;
     a.sp0 = species < 0 ? 0 : species;
     a.nsp = species < 0 ? a.nspecies : 1;
@@ -294,8 +297,8 @@ void launch_tiled(ohpic_ctx *c, int mode, int strict, int species)
 {
     const TileArgs a = tile_args(c, mode, species);
     const bool f64 = c->cfg.precision == OHPIC_FP64;
-    // particles per thread per iteration: 2 in both forms (double2 / float2 vectors)
-    const int PPT = 2;
+    // particles of a group: one per thread in the FP64 form, pairs in the FP32 one
+    const int PPT = f64 ? 1 : 2;
     int64_t blocks = 0;
     if (a.sorted) {
         blocks = (int64_t)a.nsp * c->g.ntile * a.split;

@@ -51,6 +51,70 @@ __device__ __forceinline__ double split_frac(const Split &s)
     return __longlong_as_double((long long)(((unsigned long long)(p + s.e + 971) << 52) | mant));
 }
 
+// A weight in (0, 1] as an integer pair: m * 2^(e - 63) with bit 63 of m set and its
+// low 11 bits clear (53 significant bits).  Products of weights are formed and
+// rounded (to nearest, ties to even) on the integer pipes, with the bits an FP64
+// multiply gives: a multiply occupies an SM partition's FP64 pipe for 64 cycles, its
+// integer form issues about 30 instructions on pipes that are otherwise idle.
+struct Unit {
+    unsigned long long m;
+    int e;
+};
+
+// f * 2^-k for 0 < f <= 2^k, k <= 52.
+__device__ __forceinline__ Unit unit_of(unsigned long long f, int k)
+{
+    const int lz = __clzll((long long)f);
+    return Unit{f << lz, 63 - lz - k};
+}
+
+// A positive normal double.
+__device__ __forceinline__ Unit unit_of_bits(unsigned long long b)
+{
+    return Unit{((b << 11) | (1ull << 63)), (int)(b >> 52) - 1023};
+}
+
+__device__ __forceinline__ Unit unit_mul(const Unit &a, const Unit &b)
+{
+    unsigned long long hi = __umul64hi(a.m, b.m), lo = a.m * b.m;
+    const int s = (int)(hi >> 63) ^ 1;         // the product's top bit is 63 or 62
+    hi = (hi << s) | ((lo >> 63) & (unsigned long long)s);
+    lo <<= s;
+    hi |= (unsigned long long)(lo != 0);        // sticky: the low 11 bits round
+    const unsigned long long t = hi + (0x3ffull + ((hi >> 11) & 1ull));
+    Unit r;
+    r.e = a.e + b.e + 1 - s;
+    r.m = t & ~0x7ffull;
+    if (t < hi) {                               // rounded up to the next power of two
+        r.m = 1ull << 63;
+        ++r.e;
+    }
+    return r;
+}
+
+__device__ __forceinline__ double unit_double(const Unit &a)
+{
+    return __longlong_as_double((long long)(((unsigned long long)(a.e + 1022) << 52) + (a.m >> 11)));
+}
+
+// The two weights (r and 1 - r) of an axis; false when either is zero or too small for
+// the integer products (an offset that is zero or, in cell 0, below 2^-300).
+__device__ __forceinline__ bool split_units(const Split &s, Unit &r, Unit &c)
+{
+    if (s.e >= 0) {
+        const int k = 52 - s.e;
+        if (s.fr == 0) return false;
+        r = unit_of(s.fr, k);
+        c = unit_of((1ull << k) - s.fr, k);
+        return true;
+    }
+    const double x = __longlong_as_double((long long)s.fr);
+    if ((int)(s.fr >> 52) < 1023 - 300 || (long long)s.fr < 0) return false;
+    r = unit_of_bits(s.fr);
+    c = unit_of_bits((unsigned long long)__double_as_longlong(1.0 - x));   // x < 1: at least 2^-53
+    return true;
+}
+
 // round(offset * 2^48), ties up.
 __device__ __forceinline__ unsigned long long split_frac48(const Split &s)
 {

@@ -327,30 +327,6 @@ __device__ void flush_diag(const TileArgs &a, int sp, unsigned cx, unsigned cy, 
     }
 }
 
-// Register run of deposits into one staged cell; flushed when the cell changes.
-template <typename T>
-struct Run {
-    int key = -1;
-    T acc[8];
-    __device__ __forceinline__ void add(int k, const T w[8], T *srho, int sx, int sxy)
-    {
-        if (k == key) {
-#pragma unroll
-            for (int v = 0; v < 8; ++v) acc[v] += w[v];
-        } else {
-            if (key >= 0) add8(srho + key, sx, sxy, acc);
-            key = k;
-#pragma unroll
-            for (int v = 0; v < 8; ++v) acc[v] = w[v];
-        }
-    }
-    __device__ __forceinline__ void flush(T *srho, int sx, int sxy)
-    {
-        if (key >= 0) add8(srho + key, sx, sxy, acc);
-        key = -1;
-    }
-};
-
 // Sign and ">= n" tests of a double on its bit pattern (integer ALU, not the FP64
 // pipe).  lt0 is p < 0 (false for -0.0); ge is p >= n for the bits of (double)n > 0.
 __device__ __forceinline__ bool lt0(double p)
