@@ -140,7 +140,7 @@ __device__ __forceinline__ unsigned long long mul48(unsigned long long p, unsign
 }
 
 // The 8 weights of a particle whose offsets are Rx, Ry, Rz (units of 2^-48), in
-// units of 2^-48, summing to exactly 2^48; order x fastest as in add8 / deposit_global.
+// units of 2^-48, summing to exactly 2^48; order x fastest.
 __device__ __forceinline__ void fixed_weights48(int conv, unsigned long long Rx, unsigned long long Ry,
                                                 unsigned long long Rz, unsigned long long u[8])
 {

@@ -100,15 +100,15 @@ __device__ __forceinline__ void flush_box48(const TileArgs &a, const Item &it, c
 {
     const Geom &g = a.g;
     unsigned long long *w = a.wsum + (int64_t)it.sp * g.ncell;
-    const int s3 = g.sx * g.sy * g.sz;
-    for (int i = threadIdx.x; i < s3; i += blockDim.x) {
-        const unsigned long long v = ((unsigned long long)box.hi[i] << 32) | box.lo[i];
-        if (v) {
-            const int ax = i % g.sx, by = (i / g.sx) % g.sy, cz = i / (g.sx * g.sy);
-            const int x = wrapi(it.x0 - g.halo + ax, g.nx);
-            const int y = wrapi(it.y0 - g.halo + by, g.ny);
-            const int z = wrapi(it.z0 - g.halo + cz, g.nz);
-            add_checked(w + x + (int64_t)g.nx * (y + (int64_t)g.ny * z), v, a.diag);
+    const int sx = g.sx, sy = g.sy, sz = g.sz;
+    for (RowWalk r(sx, sy); r.cz < sz; r.next(sy)) {
+        const int y = wrap_near(it.y0 - g.halo + r.by, g.ny);
+        const int z = wrap_near(it.z0 - g.halo + r.cz, g.nz);
+        unsigned long long *row = w + (int64_t)g.nx * (y + (int64_t)g.ny * z);
+        const int base = sx * (r.by + sy * r.cz);
+        for (int ax = r.lane; ax < sx; ax += r.width) {
+            const unsigned long long v = ((unsigned long long)box.hi[base + ax] << 32) | box.lo[base + ax];
+            if (v) add_checked(row + wrap_near(it.x0 - g.halo + ax, g.nx), v, a.diag);
         }
     }
 }

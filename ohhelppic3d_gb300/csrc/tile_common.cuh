@@ -22,15 +22,6 @@ __device__ __forceinline__ dnode ldg_node(const dnode *p)
     r.x = a.x; r.y = a.y; r.z = b.x; r.w = b.y;
     return r;
 }
-__device__ __forceinline__ dnode lds_node(const dnode *p)
-{
-    const double2 a = ((const double2 *)p)[0], b = ((const double2 *)p)[1];
-    dnode r;
-    r.x = a.x; r.y = a.y; r.z = b.x; r.w = b.y;
-    return r;
-}
-__device__ __forceinline__ float4 lds_node(const float4 *p) { return *p; }
-
 __device__ __forceinline__ void flag_error(DevDiag *d, int code, int info)
 {
     if (atomicCAS(&d->err_code, 0, code) == 0) d->err_info = info;
@@ -65,46 +56,19 @@ __device__ __forceinline__ void cic_c(T r, T &w0, T &w1)
     }
 }
 
+// i wrapped into [0, n) by steps of n: for indices at most a few n outside, where a
+// division's latency would stall the warp.
+__device__ __forceinline__ int wrap_near(int i, int n)
+{
+    while (i < 0) i += n;
+    while (i >= n) i -= n;
+    return i;
+}
+
 __device__ __forceinline__ int wrapi(int i, int n)
 {
     i %= n;
     return i < 0 ? i + n : i;
-}
-
-__device__ __forceinline__ void atomic_add_t(float *p, float v) { atomicAdd(p, v); }
-__device__ __forceinline__ void atomic_add_t(double *p, double v) { atomicAdd(p, v); }
-__device__ __forceinline__ void atomic_add_t(unsigned long long *p, unsigned long long v) { atomicAdd(p, v); }
-
-// 8 corner contributions of one cell into a box with row pitch sx and plane pitch sxy.
-template <typename T>
-__device__ __forceinline__ void add8(T *b, int sx, int sxy, const T w[8])
-{
-    atomic_add_t(b, w[0]);
-    atomic_add_t(b + 1, w[1]);
-    atomic_add_t(b + sx, w[2]);
-    atomic_add_t(b + sx + 1, w[3]);
-    atomic_add_t(b + sxy, w[4]);
-    atomic_add_t(b + sxy + 1, w[5]);
-    atomic_add_t(b + sxy + sx, w[6]);
-    atomic_add_t(b + sxy + sx + 1, w[7]);
-}
-
-template <typename T>
-__device__ __forceinline__ void deposit_global(const Geom &g, T *rho, int ix, int iy, int iz, const T w[8])
-{
-    const int ix1 = ix + 1 == g.nx ? 0 : ix + 1;
-    const int iy1 = iy + 1 == g.ny ? 0 : iy + 1;
-    const int iz1 = iz + 1 == g.nz ? 0 : iz + 1;
-    const int64_t y0 = (int64_t)iy * g.nx, y1 = (int64_t)iy1 * g.nx;
-    const int64_t z0 = (int64_t)iz * g.nx * g.ny, z1 = (int64_t)iz1 * g.nx * g.ny;
-    atomic_add_t(rho + ix + y0 + z0, w[0]);
-    atomic_add_t(rho + ix1 + y0 + z0, w[1]);
-    atomic_add_t(rho + ix + y1 + z0, w[2]);
-    atomic_add_t(rho + ix1 + y1 + z0, w[3]);
-    atomic_add_t(rho + ix + y0 + z1, w[4]);
-    atomic_add_t(rho + ix1 + y0 + z1, w[5]);
-    atomic_add_t(rho + ix + y1 + z1, w[6]);
-    atomic_add_t(rho + ix1 + y1 + z1, w[7]);
 }
 
 // ---------------------------------------------------------------------------
@@ -123,23 +87,23 @@ template <int PPT>
 __device__ __forceinline__ bool get_item(const TileArgs &a, int64_t b, Item &it)
 {
     if (a.sorted) {
-        const int64_t per_sp = a.g.ntile * a.split;
-        const int64_t s = b / per_sp;
+        // (a launch has fewer than 2^31 items)
+        const unsigned split = (unsigned)a.split, per_sp = (unsigned)a.g.ntile * split, s = (unsigned)b / per_sp;
         it.sp = a.sp0 + (int)s;
-        const int64_t r = b - s * per_sp;
-        it.tile = (int)(r / a.split);
-        const int part = (int)(r % a.split);
+        const unsigned r = (unsigned)b - s * per_sp, ti = split == 1u ? r : r / split;
+        it.tile = (int)ti;
+        const int part = (int)(r - ti * split);
         const int64_t *tb = a.tile_begin + (int64_t)it.sp * (a.g.ntile + 1);
         const int64_t lo = tb[it.tile] / PPT;
         const int64_t hi = it.tile + 1 == a.g.ntile ? (tb[a.g.ntile] + PPT - 1) / PPT : tb[it.tile + 1] / PPT;
         const int64_t n = hi - lo;
-        it.g0 = lo + n * part / a.split;
-        it.g1 = lo + n * (part + 1) / a.split;
-        const int t = it.tile;
-        const int tx = t % a.g.ntx, ty = (t / a.g.ntx) % a.g.nty, tz = t / (a.g.ntx * a.g.nty);
+        it.g0 = split == 1u ? lo : lo + n * part / a.split;
+        it.g1 = split == 1u ? hi : lo + n * (part + 1) / a.split;
+        const unsigned row = ti / (unsigned)a.g.ntx, tz = row / (unsigned)a.g.nty;
+        const int tx = (int)(ti - row * (unsigned)a.g.ntx), ty = (int)(row - tz * (unsigned)a.g.nty);
         it.x0 = tx * a.g.tx;
         it.y0 = ty * a.g.ty;
-        it.z0 = tz * a.g.tz;
+        it.z0 = (int)tz * a.g.tz;
     } else {
         // Unsorted: consecutive chunks of every species, no staging.
         int sp = a.sp0;
@@ -168,6 +132,38 @@ __device__ __forceinline__ bool get_item(const TileArgs &a, Item &it)
 {
     return get_item<PPT>(a, (int64_t)blockIdx.x, it);
 }
+
+// Rows of a box (fixed y, z; sx nodes along x) dealt to the CTA's warps, a row to each
+// half of a warp when it fits 16 lanes.  The (y, z) of a lane's next row come by
+// addition, and indices wrap by comparison: with a division and two remainders a row,
+// the flush of a 13 x 13 x 13 box waited for them 22 times (FP32 push of 64^3 x 32 ppc
+// 307 -> 291 us, 128x128x64 1041 -> 987 us, 16^3 x 8 ppc 16.7 -> 14.7 us).
+struct RowWalk {
+    int lane, step, width, by, cz;
+    __device__ __forceinline__ RowWalk(int sx, int sy)
+    {
+        const int warp = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+        const bool two = sx <= 16;
+        width = two ? 16 : 32;
+        lane = l & (width - 1);
+        step = two ? 2 * nw : nw;
+        by = two ? 2 * warp + (l >> 4) : warp;
+        cz = 0;
+        settle(sy);
+    }
+    __device__ __forceinline__ void settle(int sy)
+    {
+        while (by >= sy) {
+            by -= sy;
+            ++cz;
+        }
+    }
+    __device__ __forceinline__ void next(int sy)
+    {
+        by += step;
+        settle(sy);
+    }
+};
 
 // Staged box: nodes (x0-halo .. x0+tx+halo) per axis, i.e. the low corners of
 // cells x0-halo .. x0+tx+halo-1 ("span" cells), so a cell with box coordinate
@@ -205,67 +201,19 @@ __device__ __forceinline__ void stage_tile(const TileArgs &a, const Item &it, No
                                            bool need_rho)
 {
     const Geom &g = a.g;
-    const int s3 = g.sx * g.sy * g.sz;
+    const int sx = g.sx, sy = g.sy, sz = g.sz, ex = min(sx, g.gx - it.x0);
     const NodeT *E = (const NodeT *)a.epad;
-    for (int i = threadIdx.x; i < s3; i += blockDim.x) {
-        if (need_e) {
-            const int ax = i % g.sx, by = (i / g.sx) % g.sy, cz = i / (g.sx * g.sy);
+    if (need_e)
+        for (RowWalk r(sx, sy); r.cz < sz; r.next(sy)) {
             // padded index of node (x0 - halo + ax) is x0 + ax; the box of a last tile
             // that is shorter than the others reaches past the array
-            if (it.x0 + ax < g.gx && it.y0 + by < g.gy && it.z0 + cz < g.gz)
-                sE[i] = ldg_node(E + ((int64_t)(it.z0 + cz) * g.gy + (it.y0 + by)) * g.gx + (it.x0 + ax));
+            if (it.z0 + r.cz >= g.gz || it.y0 + r.by >= g.gy) continue;
+            const NodeT *src = E + ((int64_t)(it.z0 + r.cz) * g.gy + (it.y0 + r.by)) * g.gx + it.x0;
+            const int base = sx * (r.by + sy * r.cz);
+            for (int ax = r.lane; ax < ex; ax += r.width) sE[base + ax] = ldg_node(src + ax);
         }
-        if (need_rho) srho[i] = T(0);
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void flush_tile(const TileArgs &a, const Item &it, const T *srho)
-{
-    const Geom &g = a.g;
-    const int s3 = g.sx * g.sy * g.sz;
-    T *rho = (T *)a.rho;
-    for (int i = threadIdx.x; i < s3; i += blockDim.x) {
-        const T v = srho[i];
-        if (v != T(0)) {
-            const int ax = i % g.sx, by = (i / g.sx) % g.sy, cz = i / (g.sx * g.sy);
-            const int x = wrapi(it.x0 - g.halo + ax, g.nx);
-            const int y = wrapi(it.y0 - g.halo + by, g.ny);
-            const int z = wrapi(it.z0 - g.halo + cz, g.nz);
-            atomic_add_t(rho + x + (int64_t)g.nx * (y + (int64_t)g.ny * z), v);
-        }
-    }
-}
-
-// E nodes of the cell with low corner (ix, iy, iz): from the staged box when key >= 0.
-template <typename NodeT>
-__device__ __forceinline__ void load_nodes(const TileArgs &a, const Box &b, int key, int ix, int iy, int iz,
-                                           const NodeT *sE, NodeT nd[8])
-{
-    if (key >= 0) {
-        const NodeT *p = sE + key;
-        nd[0] = lds_node(p);
-        nd[1] = lds_node(p + 1);
-        nd[2] = lds_node(p + b.sx);
-        nd[3] = lds_node(p + b.sx + 1);
-        nd[4] = lds_node(p + b.sxy);
-        nd[5] = lds_node(p + b.sxy + 1);
-        nd[6] = lds_node(p + b.sxy + b.sx);
-        nd[7] = lds_node(p + b.sxy + b.sx + 1);
-    } else {
-        const Geom &g = a.g;
-        const NodeT *E = (const NodeT *)a.epad;
-        const int64_t gxy = (int64_t)g.gx * g.gy;
-        const NodeT *p = E + (ix + g.halo) + (int64_t)g.gx * (iy + g.halo) + gxy * (iz + g.halo);
-        nd[0] = ldg_node(p);
-        nd[1] = ldg_node(p + 1);
-        nd[2] = ldg_node(p + g.gx);
-        nd[3] = ldg_node(p + g.gx + 1);
-        nd[4] = ldg_node(p + gxy);
-        nd[5] = ldg_node(p + gxy + 1);
-        nd[6] = ldg_node(p + gxy + g.gx);
-        nd[7] = ldg_node(p + gxy + g.gx + 1);
-    }
+    if (need_rho)
+        for (int i = threadIdx.x; i < sx * sy * sz; i += blockDim.x) srho[i] = T(0);
 }
 
 // Block-wide reduction of the per-thread diagnostics into DevDiag.  The counts
