@@ -215,7 +215,7 @@ int grid_for(int64_t n, int threads)
 // that is nearly empty, or that do not fill the first one, wastes the rest.  The
 // split with the least waves x (cost of one CTA) is taken, a CTA costing a fixed
 // part (its boxes, its first loads) and a part per particle, both measured:
-// FP32 18 us + 3.7 ns, FP64 8 us + 32 ns.  A push of 48^3 x 16 ppc in FP64 (432
+// FP32 18 us + 3.7 ns, FP64 8 us + 27 ns.  A push of 48^3 x 16 ppc in FP64 (432
 // tiles of 8 x 8 x 8) goes from 851 us unsplit to 695 us with two CTAs per tile;
 // 16^3 x 64 ppc from 1445 to 157 us.  A split leaves at least 256 particles to a CTA.
 int pick_split(const ohpic_ctx *c)
@@ -224,7 +224,7 @@ int pick_split(const ohpic_ctx *c)
     int64_t total = 0;
     for (int s = 0; s < c->cfg.nspecies; ++s) total += c->count[s];
     const bool f64 = c->cfg.precision == OHPIC_FP64;
-    const double fixed = f64 ? 8.0 : 18.0, per = (f64 ? 0.032 : 0.0037) * (double)total / (double)items;
+    const double fixed = f64 ? 8.0 : 18.0, per = (f64 ? 0.027 : 0.0037) * (double)total / (double)items;
     constexpr int64_t kSlots = 152 * 2;
     int best = 1;
     double least = 0.0;
@@ -321,6 +321,8 @@ void launch_tiled(ohpic_ctx *c, int mode, int strict, int species)
     // followed by the per-thread prefetch stage (7 arrays x 256 threads x 16 bytes)
     if (!f64 && a.ppl == 4) smem = (a.sorted ? ((s3 * 4 * es + s3 * 8 + 15) & ~(size_t)15) : 0) + kQuadStageBytes + 128;
     if (f64) {
+        // the boxes (whole 8-byte words, no slack) and a slot per thread and array
+        smem = (a.sorted ? (gather ? s3 * sizeof(dnode) : 0) + (dep ? s3 * 8 : 0) : 0) + kF64SlotBytes;
         launch_tiled_f64(c, a, mode, strict, blocks, smem);
         return;
     }

@@ -97,6 +97,18 @@ __device__ __forceinline__ double unit_double(const Unit &a)
     return __longlong_as_double((long long)(((unsigned long long)(a.e + 1022) << 52) + (a.m >> 11)));
 }
 
+// 1 - x for a positive normal x < 1 (its bits), rounded as the FP64 subtraction rounds
+// it: a multiple of 2^-53, exact from x = 1/2 on.
+__device__ __forceinline__ Unit unit_one_minus(unsigned long long b)
+{
+    const unsigned long long M = (b & ((1ull << 52) - 1)) | (1ull << 52);
+    const int s = min(1022 - (int)(b >> 52), 63);        // x 2^53 = M 2^-s
+    const unsigned long long q = M >> s, rem = M & ((1ull << s) - 1), half = (1ull << s) >> 1;
+    unsigned long long R = (1ull << 53) - q;             // 2^53 - x 2^53, its fraction not yet taken off
+    R -= rem > half || (rem == half && rem != 0 && (R & 1ull));
+    return unit_of(R, 53);
+}
+
 // The two weights (r and 1 - r) of an axis; false when either is zero or too small for
 // the integer products (an offset that is zero or, in cell 0, below 2^-300).
 __device__ __forceinline__ bool split_units(const Split &s, Unit &r, Unit &c)
@@ -108,10 +120,9 @@ __device__ __forceinline__ bool split_units(const Split &s, Unit &r, Unit &c)
         c = unit_of((1ull << k) - s.fr, k);
         return true;
     }
-    const double x = __longlong_as_double((long long)s.fr);
     if ((int)(s.fr >> 52) < 1023 - 300 || (long long)s.fr < 0) return false;
     r = unit_of_bits(s.fr);
-    c = unit_of_bits((unsigned long long)__double_as_longlong(1.0 - x));   // x < 1: at least 2^-53
+    c = unit_one_minus(s.fr);
     return true;
 }
 

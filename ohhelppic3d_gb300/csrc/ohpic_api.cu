@@ -61,13 +61,13 @@ int64_t tiles_of(const int n[3], const int tile[3])
 // both with one CTA per tile: 16^3 x 8 ppc 35 -> 15.8 us (4 x 4 x 4), 24^3 x 16
 // ppc 49 -> 26 us (8 x 4 x 4), 32^3 x 16 ppc 49.6 -> 37.9 us (8 x 8 x 4); FP64 at
 // 32^3 353 -> 249 us.  From 48^3 on (432 tiles) 8 x 8 x 8 is as fast as any.
-// Two CTAs must fit an SM (boxes of at most kPairNodes nodes).
+// Two CTAs must fit an SM (boxes of at most pair_nodes nodes).
 constexpr int64_t kFewTiles = 200;
 
 void default_tile(const ohpic_config &k, int halo, int tile[3])
 {
     const int n[3] = {k.nx, k.ny, k.nz};
-    const int64_t pair_nodes = k.precision == OHPIC_FP64 ? 2880 : 3540;
+    const int64_t pair_nodes = k.precision == OHPIC_FP64 ? 2580 : 3540;
     int want[3] = {8, 8, 8};
     for (int d = 0; d < 3; ++d) tile[d] = k.tile[d] > 0 ? k.tile[d] : default_edge(n[d], want[d]);
     for (int d = 2; d >= 0 && k.nspecies * tiles_of(n, tile) < kFewTiles; --d) {

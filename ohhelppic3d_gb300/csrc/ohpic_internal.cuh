@@ -31,6 +31,8 @@ constexpr int kMaxHalo = 4;
 // FP32 push with four particles per lane: per-thread prefetch stage in shared memory
 // (7 arrays x 256 threads x 16 bytes).
 constexpr size_t kQuadStageBytes = 7 * 256 * 16;
+// FP64 tile kernels: a slot per thread for each of the six particle arrays.
+constexpr size_t kF64SlotBytes = 6 * 256 * 8;
 // Warps per CTA of the tile kernels (256 threads).
 constexpr int kTileWarps = 8;
 // FP32-form deposit: CIC weights in units of 2^-24 (the 8 weights of a particle sum to exactly 2^24).

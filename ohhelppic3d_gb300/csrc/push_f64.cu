@@ -35,7 +35,7 @@
 // a warp holds for 16 cycles.  So what can be computed exactly elsewhere is: cells,
 // offsets and the deposit's weights in integers, the gather's twelve weight products
 // in integers too (f64_fixed.cuh), and the rotation without its exactly zero
-// products: 51 FP64 instructions per particle with B along z instead of 75.
+// products: 44 FP64 instructions per particle with B along z instead of 75.
 // 128x128x64 x 32 ppc x 2 species, tiles of 8 x 8 x 8, halo 2 (push, ms):
 //   two particles per thread, 64-bit shared atomics (compare-and-swap loops)  11.34
 //   + 32-bit words in the shared box                                          10.05
@@ -43,9 +43,12 @@
 //   + weight products in integers                                              8.97
 //   + one particle per thread (its loop fits the instruction cache)            7.75
 //   + no sums kept from one particle to the next (17 registers)                7.02
-// The FP64 pipe is then 79% busy.  Also tried there: every second weight product in
-// FP64 7.23, the next particle's loads issued an iteration ahead 7.01, three CTAs
-// per SM 7.81, without integer products 8.66 (one particle per thread).
+//   + 1 - x of cell 0 in integers, the kinetic sums a compile-time choice      6.54
+//   + the next particle copied to shared memory meanwhile                      5.88
+// That is 44 FP64 instructions per particle, 85% of the pipe's time.  Also tried: every
+// second weight product in FP64 7.23 (for 7.02), the next particle's loads into
+// registers an iteration ahead 7.01, three CTAs per SM 7.81, without integer products
+// 8.66 (for 7.75), the copy as a run-time choice 6.39 (for 5.88: it spills).
 #include "f64_fixed.cuh"
 #include "tile_common.cuh"
 
@@ -162,12 +165,31 @@ __device__ __forceinline__ void load_nodes3(const TileArgs &a, const Box &b, int
     nd[7] = node3(q + sxy + sx + 1, in);
 }
 
+// Particle i's words into this thread's slots (one per array, 256 threads apart).  The
+// thread reads back only what it copied, so no barrier is needed, and the copy holds
+// no registers (loaded a particle ahead into registers, the push spilled).
+template <bool VELOCITY>
+__device__ __forceinline__ void fetch_f64(double *slots, const PartF64 &p, int64_t i)
+{
+    double *s = slots + threadIdx.x;
+    copy8(s, p.x + i);
+    copy8(s + 256, p.y + i);
+    copy8(s + 512, p.z + i);
+    if (VELOCITY) {
+        copy8(s + 768, p.vx + i);
+        copy8(s + 1024, p.vy + i);
+        copy8(s + 1280, p.vz + i);
+    }
+}
+
 // Which components of B are zero on the whole grid: the Boris rotation's products with
 // a zero component are exact zeros, so leaving them out gives the same bits with
 // 8 (B along z) or no FP64 operations instead of 18.
 enum Rotation { ROT_FULL, ROT_Z, ROT_NONE };
 
-template <int MODE, bool STRICT, int ROT = ROT_FULL>
+// ENERGY: the push keeps the kinetic sums (a.with_energy); as a run-time choice their
+// six FP64 instructions were issued, predicated off, for every particle.
+template <int MODE, bool STRICT, int ROT = ROT_FULL, bool ENERGY = false>
 __global__ void __launch_bounds__(256, 2) tiled_f64(TileArgs a, PartF64 p)
 {
     using Ops = typename std::conditional<STRICT, StrictOps, FastOps>::type;
@@ -182,6 +204,10 @@ __global__ void __launch_bounds__(256, 2) tiled_f64(TileArgs a, PartF64 p)
     extern __shared__ __align__(32) unsigned char smem[];
     const int s3 = g.sx * g.sy * g.sz;
     dnode *sE = (dnode *)smem;
+    // the next particle's coordinates and velocities, copied while this one is computed
+    double *next = (double *)(smem + (box.on ? (kGather ? (size_t)s3 * sizeof(dnode) : 0) + (kDeposit ? (size_t)s3 * 8 : 0)
+                                             : 0));
+    if (it.g0 + threadIdx.x < it.g1) fetch_f64<kGather>(next, p, it.g0 + threadIdx.x);
     Box48 sbox;
     sbox.lo = (unsigned *)(smem + (kGather ? (size_t)s3 * sizeof(dnode) : 0));
     sbox.hi = sbox.lo + s3;
@@ -199,12 +225,15 @@ __global__ void __launch_bounds__(256, 2) tiled_f64(TileArgs a, PartF64 p)
     unsigned long long *wsum = a.wsum + (int64_t)sp * g.ncell;
 
     for (int64_t i = it.g0 + threadIdx.x; i < it.g1; i += blockDim.x) {
-        double x = p.x[i], y = p.y[i], z = p.z[i], vx = 0.0, vy = 0.0, vz = 0.0;
+        copies_landed();
+        const double *own = next + threadIdx.x;
+        double x = own[0], y = own[256], z = own[512], vx = 0.0, vy = 0.0, vz = 0.0;
         if (kGather) {
-            vx = p.vx[i];
-            vy = p.vy[i];
-            vz = p.vz[i];
+            vx = own[768];
+            vy = own[1024];
+            vz = own[1280];
         }
+        if (i + blockDim.x < it.g1) fetch_f64<kGather>(next, p, i + blockDim.x);
         if (kGather) {
             Split sx_, sy_, sz_;
             const int ix = split_cell(x, sx_), iy = split_cell(y, sy_), iz = split_cell(z, sz_);
@@ -339,7 +368,7 @@ __global__ void __launch_bounds__(256, 2) tiled_f64(TileArgs a, PartF64 p)
                         if (ge_bits(z, bnz)) z = Ops::sub(z, fnz);
                     }
                 }
-                if (a.with_energy) {
+                if (ENERGY) {
                     ke = fma(vx, vx, fma(vy, vy, fma(vz, vz, ke)));
                     px += vx; py += vy; pz += vz;
                 }
@@ -387,6 +416,14 @@ static void launch_k(ohpic_ctx *c, void (*kernel)(TileArgs, P), const TileArgs &
     ++c->launches;
 }
 
+template <bool ENERGY>
+static auto push_kernel(bool xy_zero, double bz)
+{
+    return !xy_zero    ? tiled_f64<MODE_PUSH, false, ROT_FULL, ENERGY>
+           : bz != 0.0 ? tiled_f64<MODE_PUSH, false, ROT_Z, ENERGY>
+                       : tiled_f64<MODE_PUSH, false, ROT_NONE, ENERGY>;
+}
+
 void launch_tiled_f64(ohpic_ctx *c, const TileArgs &a, int mode, int strict, int64_t blocks, size_t smem)
 {
     const PartF64 &pp = c->p64[c->cur];
@@ -395,14 +432,18 @@ void launch_tiled_f64(ohpic_ctx *c, const TileArgs &a, int mode, int strict, int
     case MODE_PUSH * 2: {
         const double *b = c->cfg.b0;
         const bool xy = b[0] == 0.0 && b[1] == 0.0;
-        launch_k(c,
-                 !xy            ? tiled_f64<MODE_PUSH, false, ROT_FULL>
-                 : b[2] != 0.0 ? tiled_f64<MODE_PUSH, false, ROT_Z>
-                               : tiled_f64<MODE_PUSH, false, ROT_NONE>,
-                 a, blocks, smem, pp);
+        if (a.with_energy)
+            launch_k(c, push_kernel<true>(xy, b[2]), a, blocks, smem, pp);
+        else
+            launch_k(c, push_kernel<false>(xy, b[2]), a, blocks, smem, pp);
         break;
     }
-    case MODE_MOVE * 2 + 1: launch_k(c, tiled_f64<MODE_MOVE, true>, a, blocks, smem, pp); break;
+    case MODE_MOVE * 2 + 1:
+        if (a.with_energy)
+            launch_k(c, tiled_f64<MODE_MOVE, true, ROT_FULL, true>, a, blocks, smem, pp);
+        else
+            launch_k(c, tiled_f64<MODE_MOVE, true>, a, blocks, smem, pp);
+        break;
     case MODE_DEPOSIT * 2:
     case MODE_DEPOSIT * 2 + 1: launch_k(c, tiled_f64<MODE_DEPOSIT, false>, a, blocks, smem, pp); break;
     case MODE_INTERP * 2 + 1: launch_k(c, tiled_f64<MODE_INTERP, true>, a, blocks, smem, pp); break;

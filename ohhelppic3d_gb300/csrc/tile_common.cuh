@@ -25,6 +25,11 @@ __device__ __forceinline__ void copy16(void *dst, const void *src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
 }
+__device__ __forceinline__ void copy8(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 __device__ __forceinline__ void copy_node(float4 *dst, const float4 *src) { copy16(dst, src); }
 __device__ __forceinline__ void copy_node(dnode *dst, const dnode *src)
 {

@@ -31,6 +31,16 @@ def _unit_mul(a, b):
     return (1 << 63, e + 1) if t < hi else (t & ~0x7ff, e)
 
 
+def _one_minus(x: float):
+    b = int(np.float64(x).view(np.uint64))
+    M, s = (b & ((1 << 52) - 1)) | (1 << 52), min(1022 - (b >> 52), 63)
+    q, rem, half = M >> s, M & ((1 << s) - 1), (1 << s) >> 1
+    R = (1 << 53) - q
+    R -= rem > half or (rem == half and rem != 0 and R & 1)
+    lz = 64 - R.bit_length()
+    return R << lz, 63 - lz - 53
+
+
 def _double(u) -> float:
     return float(np.ldexp(float(u[0] >> 11), u[1] - 52))
 
@@ -45,6 +55,9 @@ def test_integer_weight_products_are_the_fp64_ones():
         ab = _unit_mul(_unit(a), _unit(b))
         assert _double(ab) == a * b
         assert _double(_unit_mul(ab, _unit(c))) == (a * b) * c
+    for x in np.concatenate([r, [0.5, 0.25, np.nextafter(0.5, 0), np.nextafter(0.5, 1), np.nextafter(1, 0), 2.0 ** -53,
+                                 2.0 ** -54, 3 * 2.0 ** -54, 2.0 ** -300, 1.5 * 2.0 ** -53]]):
+        assert _double(_one_minus(float(x))) == 1.0 - x, x
     # ties: (1 + 2^-27)(1 + 2^-26) / 4 has 54 significant bits
     for k in range(1, 60):
         a, b = (1 + k * 2.0 ** -27) / 2, (1 + 2.0 ** -26) / 2
