@@ -154,7 +154,8 @@ struct Run {
     Geom g{};
     SpeciesConst sc[OHPIC_MAX_SPECIES]{};
     int64_t steps = 0;
-    int64_t items = 0;
+    int64_t items = 0;            // (species, tile) pairs
+    int split = 1;                // queue items each of them is cut into
     double t_submit = 0, t_admit = 0, t_finish = 0;
     int status = OHPIC_OK;
     bool done = false;
@@ -439,7 +440,7 @@ RunDesc make_desc(const Server *s, const Run *r)
     a.g = r->g;
     a.nspecies = r->nsp;
     a.weights = s->cfg.weights;
-    a.split = 1;
+    a.split = r->split;
     a.deposit = s->cfg.deposit;
     a.use_tma = 0;
     a.with_energy = 0;
@@ -477,14 +478,49 @@ void stage_done(Server *s, int slot)
     s->stage_used[slot] = true;
 }
 
+double per_item(const Run *r) { return (double)r->total / (double)std::max<int64_t>(r->items * r->split, 1); }
+
+int parts_of(const Run *r, int64_t most)
+{
+    const int64_t per = std::max<int64_t>(r->items, 1) * most;
+    return (int)std::max<int64_t>((r->total + per - 1) / per, 1);
+}
+
+// Cuts every run's tiles into items of at most so many particles that the queue's end
+// is early: the work shared by the CTAs' slots, plus half of the longest item, which
+// the last slot still runs while the others wait.  An item costs what the single
+// context's CTA does (18 us + 3.7 ns a particle).  A queue that is long against its items
+// stays whole (two runs of 64^3 x 64 ppc: 1554 to 1574 us a tick whole, 1578 in halves); a few
+// runs, or the last of many, do not fill the chip with whole tiles: a tick of one run
+// of 16^3 x 64 ppc goes from 271 to 80 us, of 32^3 x 32 ppc from 239 to 128.
+void split_items(std::vector<Run *> &runs, int64_t slots)
+{
+    constexpr double kFixed = 18.0, kPer = 0.0037;
+    double least = 0.0;
+    int64_t best = 0;
+    for (int64_t most = 1 << 18; most >= 1 << 10; most >>= 1) {
+        double work = 0.0, longest = 0.0;
+        for (const Run *r : runs) {
+            const int parts = parts_of(r, most);
+            const double cost = kFixed + kPer * (double)r->total / (double)std::max<int64_t>(r->items * parts, 1);
+            work += cost * (double)(r->items * parts);
+            longest = std::max(longest, cost);
+        }
+        const double end = work / (double)slots + 0.5 * longest;
+        if (best == 0 || end < least) {
+            least = end;
+            best = most;
+        }
+    }
+    for (Run *r : runs) r->split = parts_of(r, best);
+}
+
 // Uploads the tables of `runs` (in queue order: decreasing particles per item)
 // and the slot masks of every pool.  Sets the launch shapes.
 bool upload_tables(Server *s, std::vector<Run *> &runs)
 {
-    std::stable_sort(runs.begin(), runs.end(), [](const Run *x, const Run *y) {
-        return (double)x->total / (double)std::max<int64_t>(x->items, 1) >
-               (double)y->total / (double)std::max<int64_t>(y->items, 1);
-    });
+    split_items(runs, (int64_t)s->sms * 2);
+    std::stable_sort(runs.begin(), runs.end(), [](const Run *x, const Run *y) { return per_item(x) > per_item(y); });
     const int n = (int)runs.size();
     int nseg = 0;
     for (const Run *r : runs) nseg += r->nsp;
@@ -509,7 +545,7 @@ bool upload_tables(Server *s, std::vector<Run *> &runs)
     for (int i = 0; i < n; ++i) {
         Run *r = runs[i];
         hr[i] = make_desc(s, r);
-        items += r->items;
+        items += r->items * r->split;
         he[i] = items;
         parts += r->total;
         max_nt = std::max<int64_t>(max_nt, r->g.ntile);
