@@ -77,7 +77,7 @@ typedef struct ohpic_config {
     int32_t precision;          /* OHPIC_FP64 or OHPIC_FP32 */
     int32_t weights;            /* OHPIC_WEIGHTS_* */
     int32_t sort_every;         /* cell sort cadence in steps; 0 = only explicit ohpic_sort */
-    int32_t tile[3];            /* tile shape in cells; 0 = tuned default */
+    int32_t tile[3];            /* tile shape in cells; 0 = a default for the grid and the species */
     int32_t track_ids;          /* 1: keep a per-particle id through sorts */
     int32_t device;             /* CUDA device ordinal */
     double dt;                  /* default time step (parameters.f90:213) */
@@ -262,7 +262,8 @@ enum {
                                      atomics cost less than the shuffles) */
 };
 typedef struct ohpic_tuning {
-    int32_t tile[3];            /* cells per tile edge; powers of two dividing n, <= 64 */
+    int32_t tile[3];            /* cells per tile edge, <= 64: divisors of n, or the default edge (the
+                                   last tile of an axis may then be shorter) */
     int32_t halo;               /* cells staged around a tile, 0..4 */
     int32_t split;              /* CTAs per (species, tile), 1..64 */
     int32_t deposit;            /* OHPIC_DEPOSIT_* (FP32 form) */

@@ -4,10 +4,10 @@
  * (src/ohhelppic3d.f90:311-358).  The server accepts independent runs while
  * others are on the GPU.  Each run is admitted by its HBM footprint, and every
  * admitted run is advanced one step per tick:
- *   - the fields of all runs of one grid size are solved together: batched
- *     cuFFT plus pooled kernels over the size class's field slots;
+ *   - the fields of all runs of one grid size are solved together over the size
+ *     class's field slots, the size classes side by side;
  *   - the particles of all runs are pushed by one persistent kernel that pulls
- *     (run, species, tile) items from a shared queue;
+ *     items, (run, species, tile) or a part of one, from a shared queue;
  *   - the cell sort of all runs is one histogram, one scan and one scatter.
  * A tick is captured once into a CUDA graph and replayed until the set of
  * runs changes.
@@ -17,7 +17,7 @@
  * other runs share the GPU:
  *   - the deposit is integer fixed point;
  *   - every particle is advanced independently;
- *   - a slot's transform is the same batched plan whatever the other slots hold.
+ *   - a slot's transform is the same whatever the other slots hold.
  *
  * Threading: one worker thread per server drives the GPU.  submit, poll,
  * result, wait and stats may be called from any host thread.

@@ -5,11 +5,13 @@
 // run resident and advances all of them one step per tick:
 //
 //   fields     runs of one grid size share a FieldPool (fields.cu): slot k of the
-//              pool is one run's rho/phi/spectrum/padded E/weight sums.  One batched
-//              cuFFT plan pair and three pooled kernels solve every slot at once.
+//              pool is one run's rho/phi/spectrum/padded E/weight sums.  Four kernels
+//              (spectral.cu; for grids whose planes do not fit shared memory, a batched
+//              cuFFT plan pair and three pooled kernels) solve every slot at once, and
+//              the pools of a tick are solved side by side.
 //   particles  one persistent launch of tiled_f32_multi (push_f32.cu) over all
-//              runs: CTAs pull (run, species, tile) items from one queue ordered
-//              by decreasing particles per item.
+//              runs: CTAs pull (run, species, tile) items, cut into parts when the
+//              queue is short, from one queue ordered by decreasing particles per item.
 //   sort       every sort_every ticks, one histogram, one scan, one record scatter
 //              and one transpose over every (run, species) segment (sort.cu); the
 //              counters of all segments live in one key space laid out by pool slot.
@@ -31,8 +33,8 @@
 // freed once the host has copied the result.
 //
 // Independence: the deposit is integer fixed point, every particle advances on
-// its own, and a slot's transform is the same batched plan whatever the other
-// slots hold, so a run's arrays do not depend on its neighbours or its slot.
+// its own, and a slot's transform is the same whatever the other slots hold, so a
+// run's arrays do not depend on its neighbours, its slot or how its tiles are cut.
 // Only FP64 atomic sums (charge, energies) may differ in the last bits.
 #include <cuda_runtime.h>
 #include <cufft.h>

@@ -30,14 +30,6 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;                      // per thread
 constexpr int kScanBlock = kScanThreads * kScanItems;
 
-__device__ __forceinline__ uint32_t tile_key(const Geom &g, int ix, int iy, int iz)
-{
-    const int tx = ix / g.tx, ty = iy / g.ty, tz = iz / g.tz;
-    const int lx = ix - tx * g.tx, ly = iy - ty * g.ty, lz = iz - tz * g.tz;
-    const uint32_t tile = (uint32_t)tx + (uint32_t)g.ntx * ((uint32_t)ty + (uint32_t)g.nty * (uint32_t)tz);
-    return tile * (uint32_t)g.tile_cells + (uint32_t)lx + (uint32_t)g.tx * ((uint32_t)ly + (uint32_t)g.ty * lz);
-}
-
 // The tile-major key is a sum of one term per axis: with tile (TX, TY, TZ),
 //   key = [ (ix/TX) C + ix%TX ] + [ (iy/TY) NTX C + TX (iy%TY) ] + [ (iz/TZ) NTX NTY C + TX TY (iz%TZ) ]
 // (C = cells per tile, NTX/NTY tiles per row/plane), so the single-context sort
@@ -59,16 +51,15 @@ __global__ void k_key_table(Geom g, uint32_t *tab)
     }
 }
 
-// Key of cell (ix, iy, iz) from the table when there is one, else by division;
-// a cell outside the grid flags OHPIC_ERR_BOUNDS and sorts as cell 0.
+// Key of cell (ix, iy, iz) from the table; a cell outside the grid flags
+// OHPIC_ERR_BOUNDS and sorts as cell 0.
 __device__ __forceinline__ uint32_t cell_key(const Geom &g, const uint32_t *tab, int ix, int iy, int iz, DevDiag *d)
 {
     if ((unsigned)ix >= (unsigned)g.nx || (unsigned)iy >= (unsigned)g.ny || (unsigned)iz >= (unsigned)g.nz) {
         if (atomicCAS(&d->err_code, 0, OHPIC_ERR_BOUNDS) == 0) d->err_info = 10;
         ix = iy = iz = 0;
     }
-    if (tab) return __ldg(tab + ix) + __ldg(tab + g.nx + iy) + __ldg(tab + g.nx + g.ny + iz);
-    return tile_key(g, ix, iy, iz);
+    return __ldg(tab + ix) + __ldg(tab + g.nx + iy) + __ldg(tab + g.nx + g.ny + iz);
 }
 
 // FP32 form, sort lead h > 0 (cells per unit velocity): a particle is filed
@@ -654,7 +645,7 @@ __device__ __forceinline__ int find_seg(const int32_t *s_end, int nseg, int64_t 
 }
 
 // Keys of one segment's grid.  The server's tiles are powers of two that divide the
-// grid, so tile_key's divisions are shifts.
+// grid, so the tile and the cell within it are shifts and masks.
 struct SegKeys {
     int n[3], ntx, nty, lx, ly, lz;
     float h;
