@@ -42,10 +42,12 @@ namespace ohpic {
 namespace {
 
 // The launch shape the autotuner picks for the dense plasmas (tile 16 x 8 x 8
-// cells, halo 2) has its own push kernels with the box geometry fixed at
-// compile time: node offsets become immediates of the shared-memory loads and
-// atomics instead of registers and adds.
-constexpr int kFixTx = 16, kFixTy = 8, kFixTz = 8, kFixHalo = 2;
+// cells, halo 2) and the default one (8 x 8 x 8) have their own push kernels with
+// the box geometry fixed at compile time: node offsets become immediates of the
+// shared-memory loads and atomics instead of registers and adds (default shape:
+// 64^3 x 32 ppc 289 -> 283 us a push, 64 x 64 x 256 x 16 575 -> 554, 128 x 128 x 64
+// x 32 980 -> 961).
+constexpr int kFixTy = 8, kFixTz = 8, kFixHalo = 2;
 
 // Segmented sum of u over runs of equal keys held by adjacent lanes (at most 5
 // shuffle steps, stopping early when the runs are short); returns true in the
@@ -770,7 +772,7 @@ __device__ __forceinline__ void tile_pass(const TileArgs &a, const PartF32 &p, c
 // the lanes' last sums once per 128 particles.  The per-particle arithmetic is
 // advance_pair(), as in the two-per-lane pass, and every sum is integer, so both
 // passes give the same bits.
-template <int MODE, int DEP, int W, bool REC = false, bool FIX = false>
+template <int MODE, int DEP, int W, bool REC = false, int FIX = 0>
 __device__ __forceinline__ void tile_pass4(const TileArgs &a, const PartF32 &p, const CUtensorMap *emap,
                                            const Item &it, unsigned char *smem, uint64_t *ebar,
                                            const RecIn &rin = RecIn{})
@@ -782,12 +784,12 @@ __device__ __forceinline__ void tile_pass4(const TileArgs &a, const PartF32 &p, 
 
     const Geom &g = a.g;
     Box box = make_box(g, it);
-    if constexpr (FIX) {
-        // the box of tile (16,8,8) with halo 2, its spans and pitches immediates
-        box.spx = kFixTx + 2 * kFixHalo;
+    if constexpr (FIX > 0) {
+        // the box of tile (FIX,8,8) with halo 2, its spans and pitches immediates
+        box.spx = FIX + 2 * kFixHalo;
         box.spy = kFixTy + 2 * kFixHalo;
         box.spz = kFixTz + 2 * kFixHalo;
-        box.sx = kFixTx + 2 * kFixHalo + 1;
+        box.sx = FIX + 2 * kFixHalo + 1;
         box.sxy = box.sx * (kFixTy + 2 * kFixHalo + 1);
     }
     const int s3 = FIX ? box.sxy * (kFixTz + 2 * kFixHalo + 1) : g.sx * g.sy * g.sz;
@@ -903,7 +905,7 @@ __device__ __forceinline__ unsigned char *align128(unsigned char *p)
 }
 
 // Work item b with PPL particles per lane: 2 (every mode) or 4 (push and deposit).
-template <int MODE, int DEP, int PPL, int W, bool FIX = false>
+template <int MODE, int DEP, int PPL, int W, int FIX = 0>
 __device__ __forceinline__ void run_item(const TileArgs &a, const PartF32 &p, const CUtensorMap *emap, int64_t b,
                                          unsigned char *smem, uint64_t *ebar)
 {
@@ -915,9 +917,9 @@ __device__ __forceinline__ void run_item(const TileArgs &a, const PartF32 &p, co
     }
 }
 
-// One context: one CTA per work item.  FIX: the launch's tile is (16,8,8) with
+// One context: one CTA per work item.  FIX > 0: the launch's tile is (FIX,8,8) with
 // halo 2, so the box spans and pitches are compile-time constants.
-template <int MODE, int DEP, int PPL, int W, bool FIX = false>
+template <int MODE, int DEP, int PPL, int W, int FIX = 0>
 __global__ void __launch_bounds__(256, 2) tiled_f32(TileArgs a, PartF32 p, const __grid_constant__ CUtensorMap emap)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -928,7 +930,7 @@ __global__ void __launch_bounds__(256, 2) tiled_f32(TileArgs a, PartF32 p, const
 
 // The push right after a sort, reading the sort's records (four per lane, LANES
 // deposit: the default launch shape); writes the word arrays p and the ids.
-template <int W, bool FIX>
+template <int W, int FIX>
 __global__ void __launch_bounds__(256, 2) tiled_f32_rec(TileArgs a, PartF32 p, RecIn rin,
                                                         const __grid_constant__ CUtensorMap emap)
 {
@@ -1040,12 +1042,14 @@ void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks,
 {
     const PartF32 &pp = c->p32[c->cur];
     const Geom &g = a.g;
-    const bool fix = g.tx == kFixTx && g.ty == kFixTy && g.tz == kFixTz && g.halo == kFixHalo;
+    const int fix = g.ty == kFixTy && g.tz == kFixTz && g.halo == kFixHalo && (g.tx == 8 || g.tx == 16) ? g.tx : 0;
     by_weights(a.weights, [&](auto w) {
         constexpr int W = decltype(w)::value;
         if (rin) {
             if (blocks <= 0) return 0;
-            auto kernel = fix ? tiled_f32_rec<W, true> : tiled_f32_rec<W, false>;
+            auto kernel = fix == 16  ? tiled_f32_rec<W, 16>
+                          : fix == 8 ? tiled_f32_rec<W, 8>
+                                     : tiled_f32_rec<W, 0>;
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (smem > 96 * 1024)
                 cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1058,8 +1062,11 @@ void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks,
             by_lanes(a.ppl, [&](auto l) {
                 return by_deposit(a.deposit, [&](auto d) {
                     constexpr int D = decltype(d)::value, L = decltype(l)::value;
-                    if (mode == MODE_PUSH && L == 4 && D == OHPIC_DEPOSIT_LANES && fix)
-                        launch_k(c, tiled_f32<MODE_PUSH, D, L, W, true>, a, blocks, smem, pp);
+                    constexpr bool kFixed = L == 4 && D == OHPIC_DEPOSIT_LANES;
+                    if (mode == MODE_PUSH && kFixed && fix == 16)
+                        launch_k(c, tiled_f32<MODE_PUSH, D, L, W, kFixed ? 16 : 0>, a, blocks, smem, pp);
+                    else if (mode == MODE_PUSH && kFixed && fix == 8)
+                        launch_k(c, tiled_f32<MODE_PUSH, D, L, W, kFixed ? 8 : 0>, a, blocks, smem, pp);
                     else if (mode == MODE_PUSH) launch_k(c, tiled_f32<MODE_PUSH, D, L, W>, a, blocks, smem, pp);
                     else launch_k(c, tiled_f32<MODE_DEPOSIT, D, L, W>, a, blocks, smem, pp);
                     return 0;
