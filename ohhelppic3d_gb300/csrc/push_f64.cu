@@ -45,7 +45,7 @@
 //   + no sums kept from one particle to the next (17 registers)                7.02
 //   + 1 - x of cell 0 in integers, the kinetic sums a compile-time choice      6.54
 //   + the next particle copied to shared memory meanwhile                      5.88
-// That is 44 FP64 instructions per particle, 85% of the pipe's time.  Also tried: every
+// That is 44 FP64 instructions per particle, 82% of the pipe's time.  Also tried: every
 // second weight product in FP64 7.23 (for 7.02), the next particle's loads into
 // registers an iteration ahead 7.01, three CTAs per SM 7.81, without integer products
 // 8.66 (for 7.75), the copy as a run-time choice 6.39 (for 5.88: it spills).
