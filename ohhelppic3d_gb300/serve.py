@@ -266,7 +266,8 @@ class Server:
             fields = np.empty(5 * int(np.prod(req.n)), dtype=np.float64)
             fp = fields.ctypes.data_as(_DP)
         if req is not None and req.keep_particles:
-            parts = np.empty(6 * req.particles(), dtype=np.float64)
+            # the injector rounds a species' fractional count up or down by a draw
+            parts = np.empty(6 * (req.particles() + len(req.species)), dtype=np.float64)
             pp = parts.ctypes.data_as(_DP)
         self._check(self.L.ohpic_serve_result(self.h, rid, C.byref(res), fp, pp), "result")
         d = res.diag
