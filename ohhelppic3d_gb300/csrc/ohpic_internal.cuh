@@ -146,6 +146,7 @@ constexpr int kMaxServeRuns = 512;
 struct RunDesc {
     TileArgs a;
     PartF32 p;
+    RecIn rin;   // the sort's records (launch_multi_f32 with records)
 };
 // Arguments of the multi-run persistent push: runs[r] owns the items
 // [item_end[r-1], item_end[r]) of one queue; cursor is zero at launch.  The run
@@ -322,7 +323,7 @@ void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks,
 // other than the push that consumes the records calls it first.
 void materialize_records(ohpic_ctx *c);
 cudaError_t launch_multi_f32(cudaStream_t st, int mode, int dep, int ppl, int weights, const MultiPush &m,
-                             int grid, size_t smem);
+                             int grid, size_t smem, bool records = false);
 void ensure_emap(ohpic_ctx *c);
 // Fields (fields.cu).
 int fields_setup(ohpic_ctx *c);
@@ -354,7 +355,7 @@ int scan_u32(cudaStream_t st, const uint32_t *in, uint32_t *out, int64_t n, uint
 // Multi-run sort passes; each returns the number of launches it made.
 int launch_sort_hist_multi(cudaStream_t st, const MultiSort &m, int64_t chunks);
 int launch_sort_finish_multi(cudaStream_t st, const MultiSort &m, int64_t chunks, int64_t max_ntile,
-                             int max_seg, int64_t nkeys, uint32_t *scan_tmp);
+                             int max_seg, int64_t nkeys, uint32_t *scan_tmp, bool records = false);
 // Conversions (convert.cu).
 void launch_f64_to_f32(ohpic_ctx *c, const double *stage6, int64_t n, int64_t dst, uint32_t id0,
                        int aos, int64_t stride_doubles);

@@ -12,12 +12,14 @@
 //   particles  one persistent launch of tiled_f32_multi (push_f32.cu) over all
 //              runs: CTAs pull (run, species, tile) items, cut into parts when the
 //              queue is short, from one queue ordered by decreasing particles per item.
-//   sort       every sort_every ticks, one histogram, one scan, one record scatter
-//              and one transpose over every (run, species) segment (sort.cu); the
-//              counters of all segments live in one key space laid out by pool slot.
+//   sort       every sort_every ticks, one histogram, one scan and one record scatter
+//              over every (run, species) segment (sort.cu); the counters of all
+//              segments live in one key space laid out by pool slot.  The tick's push
+//              reads the records; for a deposit (admission) and the other launch
+//              shapes a transpose writes them back into the arrays.
 //
-// A tick's launches are captured into a CUDA graph (and a second graph for the
-// sort) and replayed until the set of grid-size pools in use changes: the tables
+// A tick's launches are captured into a CUDA graph (and a tick with a sort into a
+// second) and replayed until the set of grid-size pools in use changes: the tables
 // the kernels read (run and segment counts, run descriptors, item prefix, sort
 // segments, pool slot masks) live in device memory and are refreshed by
 // stream-ordered copies from pinned staging before the tick that needs them,
@@ -462,6 +464,7 @@ RunDesc make_desc(const Server *s, const Run *r)
     a.diag = r->diag;
     a.chunk = 4096;
     d.p = r->p;
+    d.rin = RecIn{r->rec, r->ids};
     return d;
 }
 
@@ -641,7 +644,7 @@ MultiSort multi_sort(const Server *s)
 
 // The cell sort of the segments in the tables; returns launches (memsets count
 // as launches).  Grids are fixed; the kernels loop over the uploaded chunks.
-int64_t enqueue_sort(Server *s)
+int64_t enqueue_sort(Server *s, bool records)
 {
     fixed_shapes(s);
     const MultiSort m = multi_sort(s);
@@ -650,13 +653,14 @@ int64_t enqueue_sort(Server *s)
     cudaMemsetAsync(s->d_count, 0, (size_t)s->nkeys * 4, s->st);
     l += launch_sort_hist_multi(s->st, m, grid);
     cudaMemsetAsync(s->d_cur32, 0, (size_t)s->nkeys * 4, s->st);
-    l += launch_sort_finish_multi(s->st, m, grid, s->tab_max_ntile, kMaxSortSegs, s->nkeys, s->d_scan_tmp);
+    l += launch_sort_finish_multi(s->st, m, grid, s->tab_max_ntile, kMaxSortSegs, s->nkeys, s->d_scan_tmp,
+                                  records);
     return l;
 }
 
 // The field solve of every pool in use, then the push (or the deposit) of the
 // runs in the tables; returns launches, -1 on a cuFFT or launch error.
-int64_t enqueue_step(Server *s, int mode)
+int64_t enqueue_step(Server *s, int mode, bool records = false)
 {
     fixed_shapes(s);
     int64_t l = 0;
@@ -694,8 +698,7 @@ int64_t enqueue_step(Server *s, int mode)
     }
     cudaMemsetAsync(s->d_cursor, 0, sizeof(unsigned long long), s->st);
     if (launch_multi_f32(s->st, mode, s->cfg.deposit, s->cfg.lane_particles, s->cfg.weights, multi_push(s),
-                         s->push_grid,
-                         s->push_smem) != cudaSuccess)
+                         s->push_grid, s->push_smem, records) != cudaSuccess)
         return -1;
     return l + 2;
 }
@@ -909,7 +912,7 @@ bool admit(Server *s)
     // Sort, then deposit, the admitted runs only (the push of the next tick needs
     // their weight sums); the tick tables are rebuilt afterwards.
     if (!upload_tables(s, fresh)) return false;
-    const int64_t l = enqueue_sort(s);
+    const int64_t l = enqueue_sort(s, false);
     const int64_t l2 = enqueue_step(s, MODE_DEPOSIT);
     if (l2 < 0) return false;
     for (Run *r : fresh) s->active.push_back(r);
@@ -917,6 +920,16 @@ bool admit(Server *s)
     std::lock_guard<std::mutex> lk(s->mu);
     s->stats.launches += l + l2;
     return true;
+}
+
+// A tick with a sort: in the default shape of the push (four particles per lane,
+// LANES deposit) it reads the sort's records.
+int64_t enqueue_sorted_step(Server *s)
+{
+    const bool records = s->cfg.lane_particles == 4 && s->cfg.deposit == OHPIC_DEPOSIT_LANES;
+    const int64_t l = enqueue_sort(s, records);
+    const int64_t l2 = enqueue_step(s, MODE_PUSH, records);
+    return l2 < 0 ? -1 : l + l2;
 }
 
 bool capture(Server *s, bool sort, cudaGraphExec_t *out, int64_t *launches)
@@ -927,7 +940,7 @@ bool capture(Server *s, bool sort, cudaGraphExec_t *out, int64_t *launches)
     }
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(s->st, cudaStreamCaptureModeRelaxed) != cudaSuccess) return false;
-    const int64_t l = sort ? enqueue_sort(s) : enqueue_step(s, MODE_PUSH);
+    const int64_t l = sort ? enqueue_sorted_step(s) : enqueue_step(s, MODE_PUSH);
     const cudaError_t e = cudaStreamEndCapture(s->st, &g);
     if (e != cudaSuccess || l < 0 || !g) {
         if (g) cudaGraphDestroy(g);
@@ -975,18 +988,13 @@ bool tick(Server *s)
             }
         }
         if (ok && s->g_tick && s->g_sort) {
-            if (sort_now) {
-                if (cudaGraphLaunch(s->g_sort, s->st) != cudaSuccess) return false;
-                launched += s->launches_sort;
-            }
-            if (cudaGraphLaunch(s->g_tick, s->st) != cudaSuccess) return false;
-            launched += s->launches_tick;
+            if (cudaGraphLaunch(sort_now ? s->g_sort : s->g_tick, s->st) != cudaSuccess) return false;
+            launched += sort_now ? s->launches_sort : s->launches_tick;
             via_graph = true;
         }
     }
     if (!via_graph) {
-        if (sort_now) launched += enqueue_sort(s);
-        const int64_t l = enqueue_step(s, MODE_PUSH);
+        const int64_t l = sort_now ? enqueue_sorted_step(s) : enqueue_step(s, MODE_PUSH);
         if (l < 0) return false;
         launched += l;
     }
@@ -1003,7 +1011,7 @@ bool tick(Server *s)
         s->stats.sort_ticks += sort_now ? 1 : 0;
         s->stats.particle_steps += psteps;
         s->stats.launches += launched;
-        s->stats.graph_launches += via_graph ? (sort_now ? 2 : 1) : 0;
+        s->stats.graph_launches += via_graph ? 1 : 0;
     }
     // Runs that reached their step count leave after this tick.
     std::vector<Run *> keep;

@@ -832,9 +832,10 @@ int launch_sort_hist_multi(cudaStream_t st, const MultiSort &m, int64_t chunks)
 }
 
 // Scan of the key space, tile starts, then the scatter (the cursor array must be
-// zero; the caller clears it before this call).
+// zero; the caller clears it before this call).  records: the particles are left in
+// the records, for a push that reads them.
 int launch_sort_finish_multi(cudaStream_t st, const MultiSort &m, int64_t chunks, int64_t max_ntile,
-                             int max_seg, int64_t nkeys, uint32_t *scan_tmp)
+                             int max_seg, int64_t nkeys, uint32_t *scan_tmp, bool records)
 {
     int launches = scan_levels(st, m.count, m.start, nkeys, scan_tmp);
     if (max_seg > 0) {
@@ -845,8 +846,11 @@ int launch_sort_finish_multi(cudaStream_t st, const MultiSort &m, int64_t chunks
     if (chunks > 0) {
         const int64_t grid = chunks < 152 * 8 ? chunks : 152 * 8;
         k_scatter_multi<<<(unsigned)grid, 256, 0, st>>>(m);
-        k_rec32_to_soa_multi<<<(unsigned)grid, 256, 0, st>>>(m);
-        launches += 2;
+        ++launches;
+        if (!records) {
+            k_rec32_to_soa_multi<<<(unsigned)grid, 256, 0, st>>>(m);
+            ++launches;
+        }
     }
     return launches;
 }
