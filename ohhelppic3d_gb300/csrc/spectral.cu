@@ -405,13 +405,12 @@ Spectral *spectral_create(const Geom &g, const double *green)
     auto threads = [](int64_t elements) {   // about four elements per thread, whole warps
         return (int)std::min<int64_t>(std::max<int64_t>((elements / 4 + 31) / 32 * 32, 64), 512);
     };
-    auto allow = [](auto k, size_t smem) {
-        return smem <= 48 * 1024 ||
-               cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem) == cudaSuccess;
+    // (always: the 48 KB that need no opt-in hold a kernel's static shared memory too)
+    auto allow = [](auto k) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem) == cudaSuccess;
     };
-    if (!(allow(k_plane_forward<false>, plane_smem) && allow(k_plane_forward<true>, plane_smem) &&
-          allow(k_plane_inverse<false>, plane_smem) && allow(k_plane_inverse<true>, plane_smem) &&
-          allow(k_pencils, pencil_smem))) {
+    if (!(allow(k_plane_forward<false>) && allow(k_plane_forward<true>) && allow(k_plane_inverse<false>) &&
+          allow(k_plane_inverse<true>) && allow(k_pencils))) {
         cudaGetLastError();
         cudaFree(tw);
         return nullptr;
