@@ -33,6 +33,20 @@ constexpr int kMaxHalo = 4;
 constexpr size_t kQuadStageBytes = 7 * 256 * 16;
 // FP64 tile kernels: a slot per thread for each of the six particle arrays.
 constexpr size_t kF64SlotBytes = 6 * 256 * 8;
+// The largest boxes (E and deposit) a tile shape may have, and the dynamic shared memory
+// that every tile kernel may be launched with.
+constexpr size_t kMaxBoxBytes = 192 * 1024;
+constexpr size_t kTileShared = kMaxBoxBytes + kQuadStageBytes + 128;
+
+// Opts a tile kernel in to kTileShared.  Made for every launch: the 48 KB that need no
+// opt-in hold the kernel's static part too.  Always the same value: the limit belongs to
+// the kernel, which the contexts and servers of all threads share.
+template <typename K>
+inline cudaError_t allow_tile_shared(K *kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileShared);
+}
+
 // Warps per CTA of the tile kernels (256 threads).
 constexpr int kTileWarps = 8;
 // FP32-form deposit: CIC weights in units of 2^-24 (the 8 weights of a particle sum to exactly 2^24).

@@ -1010,7 +1010,7 @@ static void launch_k(ohpic_ctx *c, void (*kernel)(TileArgs, P, const CUtensorMap
                      int64_t blocks, size_t smem, const P &parts)
 {
     if (blocks <= 0) return;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_tile_shared(kernel);
     // CTAs over ~96 KB pair up on an SM only with the whole shared-memory carveout
     if (smem > 96 * 1024)
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1058,7 +1058,7 @@ void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks,
             auto kernel = fix == 16  ? tiled_f32_rec<W, 16>
                           : fix == 8 ? tiled_f32_rec<W, 8>
                                      : tiled_f32_rec<W, 0>;
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_tile_shared(kernel);
             if (smem > 96 * 1024)
                 cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared);
@@ -1093,8 +1093,7 @@ template <int MODE, int DEP, int PPL, int W, bool REC = false>
 static cudaError_t launch_multi_k(cudaStream_t st, const MultiPush &m, int grid, size_t smem)
 {
     auto kernel = tiled_f32_multi<MODE, DEP, PPL, W, REC>;
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_tile_shared(kernel);
     if (e != cudaSuccess) return e;
     kernel<<<(unsigned)grid, 256, smem, st>>>(m);
     return cudaGetLastError();

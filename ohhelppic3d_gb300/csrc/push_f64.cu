@@ -411,7 +411,7 @@ static void launch_k(ohpic_ctx *c, void (*kernel)(TileArgs, P), const TileArgs &
                      const P &parts)
 {
     if (blocks <= 0) return;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_tile_shared(kernel);
     kernel<<<(unsigned)blocks, 256, smem, c->stream>>>(a, parts);
     ++c->launches;
 }
