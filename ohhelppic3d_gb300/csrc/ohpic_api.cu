@@ -233,6 +233,14 @@ int do_scatter(ohpic_ctx *c)
     return OHPIC_OK;
 }
 
+// What the launches of a call that returns before its work is done came to.
+int launched(ohpic_ctx *c, const char *call)
+{
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(c, OHPIC_ERR_CUDA, std::string(call) + ": " + cudaGetErrorString(e));
+    return OHPIC_OK;
+}
+
 // The push's tallies (crossings, particles outside their tile, and the kinetic
 // sums when it tracks them): the leading bytes of DevDiag.
 size_t tally_bytes(const ohpic_ctx *c) { return c->with_energy ? offsetof(DevDiag, charge) : offsetof(DevDiag, kin); }
@@ -761,14 +769,16 @@ int ohpic_scatter(ohpic_ctx *c)
 {
     if (!c) return OHPIC_ERR_INVALID;
     cudaSetDevice(c->dev);
-    return do_scatter(c);
+    const int rc = do_scatter(c);
+    return rc == OHPIC_OK ? launched(c, "scatter") : rc;
 }
 
 int ohpic_solve(ohpic_ctx *c)
 {
     if (!c) return OHPIC_ERR_INVALID;
     cudaSetDevice(c->dev);
-    return do_solve(c);
+    const int rc = do_solve(c);
+    return rc == OHPIC_OK ? launched(c, "solve") : rc;
 }
 
 int ohpic_interp(ohpic_ctx *c, int s, double *e_out, int64_t capacity, int64_t *n_out)
@@ -814,7 +824,7 @@ int ohpic_move(ohpic_ctx *c, double dt)
     c->rho_valid = false;
     c->field_valid = false;
     c->kin_valid = false;
-    return OHPIC_OK;
+    return launched(c, "move");
 }
 
 int ohpic_push(ohpic_ctx *c, double dt)
@@ -825,7 +835,8 @@ int ohpic_push(ohpic_ctx *c, double dt)
         const int rc = do_solve(c, true);
         if (rc != OHPIC_OK) return rc;
     }
-    return do_push(c, dt);
+    const int rc = do_push(c, dt);
+    return rc == OHPIC_OK ? launched(c, "push") : rc;
 }
 
 int ohpic_sort(ohpic_ctx *c)
@@ -854,9 +865,7 @@ int ohpic_step(ohpic_ctx *c, double dt, int nsteps)
             rc = sort_particles(c);
         if (rc != OHPIC_OK) return rc;
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(c, OHPIC_ERR_CUDA, std::string("step: ") + cudaGetErrorString(e));
-    return OHPIC_OK;
+    return launched(c, "step");
 }
 
 int ohpic_download_field(ohpic_ctx *c, int which, double *host)
