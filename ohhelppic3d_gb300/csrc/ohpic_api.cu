@@ -55,6 +55,15 @@ int64_t tiles_of(const int n[3], const int tile[3])
     return nt;
 }
 
+// The widest halo that a tile's staged box has room for; -1 when none.
+int halo_room(const ohpic_config &k, const int tile[3])
+{
+    Geom g;
+    int h = kMaxHalo;
+    while (h >= 0 && !make_geom(k, tile, h, g, tile)) --h;
+    return h;
+}
+
 // Default tile of a grid: edges of about 8 cells, or of about 4 along z, then y,
 // then x while the species' tiles are too few to occupy the chip (152 SMs, two
 // CTAs each).  FP32 push, tiles of 8 x 8 x 8 against the ones this rule takes,
@@ -62,6 +71,12 @@ int64_t tiles_of(const int n[3], const int tile[3])
 // ppc 49 -> 26 us (8 x 4 x 4), 32^3 x 16 ppc 49.6 -> 37.9 us (8 x 8 x 4); FP64 at
 // 32^3 353 -> 249 us.  From 48^3 on (432 tiles) 8 x 8 x 8 is as fast as any.
 // Two CTAs must fit an SM (boxes of at most pair_nodes nodes).
+// The halo may be widened later, and the caller may have given edges of the tile: the
+// open ones shrink until the box has the room that the largest powers of two dividing the
+// axes (at most 8) leave it.  Where those have no room for the halo, they stand, and the
+// shape is refused.  FP64 push, 16 ppc, two species, against the tiles before that rule,
+// which took no halo of 4: 45^3 (9,9,5) 331 us for (9,9,8) 343, 54^3 (9,9,6) 579 for
+// (9,9,8) 546, 63^3 (9,7,7) 818 for (9,9,8) 858, 90 x 60 x 30 (9,8,6) 595 for (9,8,8) 585.
 constexpr int64_t kFewTiles = 200;
 
 void default_tile(const ohpic_config &k, int halo, int tile[3])
@@ -81,6 +96,33 @@ void default_tile(const ohpic_config &k, int halo, int tile[3])
     };
     for (int d = 2; d >= 0 && nodes() > pair_nodes; --d)
         if (k.tile[d] <= 0) tile[d] = std::min(tile[d], want[d]);
+
+    int plain[3];
+    for (int d = 0; d < 3; ++d) {
+        plain[d] = k.tile[d] > 0 ? k.tile[d] : 8;
+        while (k.tile[d] <= 0 && n[d] % plain[d]) plain[d] /= 2;
+    }
+    const int room = halo_room(k, plain);
+    if (room < halo) std::copy(plain, plain + 3, tile);
+    while (halo_room(k, tile) < room) {
+        // the widest of the edges that leave a shorter last tile, else the widest, to the next
+        // one that divides the axis, or to one equal tile more
+        int at = -1, rank = -1;
+        for (int d = 2; d >= 0; --d) {
+            const int r = tile[d] + (n[d] % tile[d] ? 64 : 0);
+            if (k.tile[d] <= 0 && tile[d] > 1 && r > rank) {
+                at = d;
+                rank = r;
+            }
+        }
+        const int t = tile[at], more = (n[at] + t - 1) / t + 1;
+        tile[at] = std::min(t - 1, (n[at] + more - 1) / more);
+        for (int e = t - 1; 2 * e >= t; --e)
+            if (n[at] % e == 0) {
+                tile[at] = e;
+                break;
+            }
+    }
 }
 
 }  // namespace
@@ -516,8 +558,11 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     const int n[3] = {k.nx, k.ny, k.nz};
     for (int d = 0; d < 3; ++d)
         if (k.tile[d] > 0 && (n[d] % k.tile[d] != 0 || k.tile[d] > 64)) return OHPIC_ERR_INVALID;
+    constexpr int kHalo = 2;
     int tile[3];
-    default_tile(k, 2, tile);
+    default_tile(k, kHalo, tile);
+    Geom shape;
+    if (!make_geom(k, tile, kHalo, shape, tile)) return OHPIC_ERR_INVALID;
 
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || k.device < 0 || k.device >= ndev) {
@@ -534,7 +579,7 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
         return OHPIC_ERR_CUDA;
     }
 
-    c->halo = 2;
+    c->halo = kHalo;
     c->split = 1;
     c->with_energy = false;
     c->sc_dt = NAN;
@@ -543,11 +588,8 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     c->sort_lead = 0;
     c->tma_polls = kTmaWaitPolls;
     Geom &g = c->g;
+    g = shape;
     for (int d = 0; d < 3; ++d) c->def_tile[d] = tile[d];
-    if (!make_geom(k, tile, c->halo, g, c->def_tile)) {
-        ohpic_destroy(c);
-        return OHPIC_ERR_INVALID;
-    }
     // sort keys of any tile this context accepts: a tile edge divides its axis or
     // is the default one, whose tiles cover at least the axis
     const int64_t nkeys = std::max(g.nkeys, g.ncell);
