@@ -265,7 +265,8 @@ typedef struct ohpic_tuning {
     int32_t tile[3];            /* cells per tile edge, <= 64: divisors of n, or the default edge (the
                                    last tile of an axis may then be shorter) */
     int32_t halo;               /* cells staged around a tile, 0..4 */
-    int32_t split;              /* CTAs per (species, tile), 1..64 */
+    int32_t split;              /* CTAs per (species, tile), 1..64; 0 (the default): chosen for each launch
+                                   so that the CTAs fill the chip, up to 16 */
     int32_t deposit;            /* OHPIC_DEPOSIT_* (FP32 form) */
     int32_t sort_every;         /* cell sort cadence in steps; 0 = only explicit sorts */
     int32_t lane_particles;     /* FP32 push: consecutive particles per lane, 2 or 4 */

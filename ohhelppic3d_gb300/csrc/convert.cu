@@ -210,7 +210,7 @@ int grid_for(int64_t n, int threads)
 
 }  // namespace
 
-// CTAs per (species, tile) when the tuning leaves it at 1: the chip runs 304 tile
+// CTAs per (species, tile) when the tuning leaves it to the library (0): the chip runs 304 tile
 // CTAs at once (two on each of 152 SMs), and a launch whose CTAs end in a wave
 // that is nearly empty, or that do not fill the first one, wastes the rest.  The
 // split with the least waves x (cost of one CTA) is taken, a CTA costing a fixed
@@ -266,7 +266,7 @@ TileArgs tile_args(ohpic_ctx *c, int mode, int species)
     a.g = c->g;
     a.nspecies = c->cfg.nspecies;
     a.weights = c->cfg.weights;
-    a.split = c->split > 1 ? c->split : pick_split(c);
+    a.split = c->split > 0 ? c->split : pick_split(c);
     a.deposit = c->dep_strategy;
     if (c->sorted && mode != MODE_DEPOSIT) ensure_emap(c);
     a.use_tma = c->sorted && c->emap_ok ? 1 : 0;

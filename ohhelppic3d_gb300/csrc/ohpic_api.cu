@@ -580,7 +580,7 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     }
 
     c->halo = kHalo;
-    c->split = 1;
+    c->split = 0;
     c->with_energy = false;
     c->sc_dt = NAN;
     c->dep_strategy = OHPIC_DEPOSIT_LANES;
@@ -1101,10 +1101,10 @@ int ohpic_get_tuning(ohpic_ctx *c, ohpic_tuning *t)
 int ohpic_set_tuning(ohpic_ctx *c, const ohpic_tuning *t)
 {
     if (!c || !t) return OHPIC_ERR_INVALID;
-    if (t->split < 1 || t->split > 64 || t->deposit < OHPIC_DEPOSIT_RUNS || t->deposit > OHPIC_DEPOSIT_LANES ||
+    if (t->split < 0 || t->split > 64 || t->deposit < OHPIC_DEPOSIT_RUNS || t->deposit > OHPIC_DEPOSIT_LANES ||
         t->sort_every < 0 || (t->lane_particles != 2 && t->lane_particles != 4))
         return fail(c, OHPIC_ERR_INVALID,
-                    "tuning: split 1..64, deposit 0..4, sort_every >= 0, lane_particles 2 or 4");
+                    "tuning: split 0..64, deposit 0..4, sort_every >= 0, lane_particles 2 or 4");
     if (t->sort_lead < 0 || t->sort_lead > 4096 || (t->sort_lead != 0 && c->cfg.precision != OHPIC_FP32))
         return fail(c, OHPIC_ERR_INVALID, "tuning: sort_lead 0..4096, nonzero only in the FP32 form");
     Geom g2;

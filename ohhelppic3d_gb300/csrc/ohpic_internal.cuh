@@ -289,7 +289,7 @@ struct ohpic_ctx {
     bool rho_valid;
     bool field_valid;
     int64_t steps;
-    int split;
+    int split;                  // CTAs per (species, tile); 0: pick_split for each launch
     int def_tile[3];            // tile the context was created with
     int halo;
     int dep_strategy;           // OHPIC_DEPOSIT_* for the FP32 warp deposit
