@@ -108,13 +108,13 @@ def tune(n, dt, b0, qm, q, capacity_per_cell, species, precision=FP32, weights=0
         return ms
 
     def fresh(cand):
-        """The push time of a candidate on the plasma as it starts."""
-        c = _ctx(cfg_kw, species)
-        try:
-            c.set_tuning(**{**best, **cand})
-            return _push_ms(c, dt, steps)
-        finally:
-            c.close()
+        """The push time of a candidate on the plasma as it starts.  The search goes on
+        there: one context at a time, as the grid itself may fill the device."""
+        nonlocal ctx
+        ctx.close()
+        ctx = _ctx(cfg_kw, species)
+        ctx.set_tuning(**{**best, **cand})
+        return _push_ms(ctx, dt, steps)
 
     def joint(candidates, duel=False):
         """Measures every candidate (a dict of tuning keys) on top of the current
