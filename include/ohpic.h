@@ -284,6 +284,8 @@ int ohpic_set_tuning(ohpic_ctx *ctx, const ohpic_tuning *tuning);
  * summed CUDA-event duration of the fused push kernel (enable first). */
 int ohpic_set_push_timing(ohpic_ctx *ctx, int enable);
 int ohpic_stats(ohpic_ctx *ctx, int64_t *launches, int64_t *push_launches, double *push_ms);
+/* Steps that ran as a replayed CUDA graph, and how often one was captured. */
+int ohpic_graph_stats(ohpic_ctx *ctx, int64_t *replays, int64_t *captures);
 /* Device bytes held by the context. */
 int ohpic_memory(ohpic_ctx *ctx, int64_t *device_bytes);
 

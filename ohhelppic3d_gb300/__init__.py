@@ -133,6 +133,7 @@ SIGNATURES = {
     "ohpic_get_stream": (C.c_int, [_P, C.POINTER(_P)]),
     "ohpic_set_push_timing": (C.c_int, [_P, C.c_int]),
     "ohpic_stats": (C.c_int, [_P, C.POINTER(C.c_int64), C.POINTER(C.c_int64), C.POINTER(C.c_double)]),
+    "ohpic_graph_stats": (C.c_int, [_P, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "ohpic_memory": (C.c_int, [_P, C.POINTER(C.c_int64)]),
     "ohpic_get_tuning": (C.c_int, [_P, C.POINTER(Tuning)]),
     "ohpic_set_tuning": (C.c_int, [_P, C.POINTER(Tuning)]),
@@ -396,6 +397,12 @@ class PicContext:
         a, b, ms = C.c_int64(), C.c_int64(), C.c_double()
         self._check(lib().ohpic_stats(self.ptr, C.byref(a), C.byref(b), C.byref(ms)))
         return {"launches": a.value, "push_launches": b.value, "push_ms": ms.value}
+
+    def graph_stats(self) -> dict:
+        """Steps that ran as a replayed CUDA graph, and how often one was captured."""
+        a, b = C.c_int64(), C.c_int64()
+        self._check(lib().ohpic_graph_stats(self.ptr, C.byref(a), C.byref(b)))
+        return {"replays": a.value, "captures": b.value}
 
     def get_tuning(self) -> dict:
         t = Tuning()

@@ -304,6 +304,7 @@ struct ohpic_ctx {
     ohpic::TileArgs step_args;
     int step_flags;
     int64_t step_launches;
+    int64_t step_replays, step_captures;
     bool step_graph_off;        // capture failed once: plain launches from then on
     bool step_launched;         // a step has been launched plainly (its kernels are loaded)
 
