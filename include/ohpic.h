@@ -329,6 +329,10 @@ int ohpic_poisson_solve(ohpic_poisson *solver, const double *rho, double *phi, d
 /* The same on device arrays, ordered on `stream` (a cudaStream_t; 0 is the
  * default stream, as everywhere in CUDA); returns without synchronising. */
 int ohpic_poisson_solve_device(ohpic_poisson *solver, const double *rho, double *phi, double *e, void *stream);
+/* How the solver transforms: pairs[i], the pairs of lines that a CTA of pass i holds (x, y
+ * forward, z both ways, y, x backward), or 0 where the block goes through cuFFT; shared[i], whether
+ * the pass copies its table to shared memory. */
+int ohpic_poisson_plan(const ohpic_poisson *solver, int32_t pairs[5], int32_t shared[5]);
 int ohpic_poisson_last_error(const ohpic_poisson *solver, char *buf, size_t len);
 
 /* CIC deposit that allocates no device memory (no counterpart in the reference).

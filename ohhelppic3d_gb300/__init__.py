@@ -144,6 +144,7 @@ SIGNATURES = {
     "ohpic_poisson_destroy": (C.c_int, [_P]),
     "ohpic_poisson_solve": (C.c_int, [_P, _DP, _DP, _DP]),
     "ohpic_poisson_solve_device": (C.c_int, [_P, _P, _P, _P, _P]),
+    "ohpic_poisson_plan": (C.c_int, [_P, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "ohpic_poisson_last_error": (C.c_int, [_P, C.c_char_p, C.c_size_t]),
 }
 
@@ -448,6 +449,13 @@ class PoissonSolver:
             buf = C.create_string_buffer(512)
             lib().ohpic_poisson_last_error(self.ptr, buf, 512)
             raise OhpicError(rc, buf.value.decode(errors="replace"))
+
+    def plan(self) -> dict:
+        """Pairs of lines per CTA and whether the table is in shared memory, per pass (x, y
+        forward, z, y, x backward); pairs of 0: the block goes through cuFFT."""
+        a, b = (C.c_int32 * 5)(), (C.c_int32 * 5)()
+        self._check(lib().ohpic_poisson_plan(self.ptr, a, b))
+        return {"pairs": tuple(a), "shared": tuple(bool(v) for v in b)}
 
     def solve(self, rho: np.ndarray, with_e: bool = True):
         rho = np.ascontiguousarray(rho, dtype=np.float64)

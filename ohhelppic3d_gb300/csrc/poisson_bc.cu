@@ -1101,6 +1101,16 @@ int ohpic_poisson_solve(ohpic_poisson *p, const double *rho, double *phi, double
     return OHPIC_OK;
 }
 
+int ohpic_poisson_plan(const ohpic_poisson *p, int32_t pairs[5], int32_t shared[5])
+{
+    if (!p || !pairs || !shared) return OHPIC_ERR_INVALID;
+    for (int i = 0; i < 5; ++i) {
+        pairs[i] = p->passes_ok ? p->pass[i].P : 0;
+        shared[i] = p->passes_ok && p->pass[i].tw_shared ? 1 : 0;
+    }
+    return OHPIC_OK;
+}
+
 int ohpic_poisson_last_error(const ohpic_poisson *p, char *buf, size_t len)
 {
     if (!p || !buf || len == 0) return OHPIC_ERR_INVALID;
