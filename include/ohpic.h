@@ -263,7 +263,8 @@ enum {
 };
 typedef struct ohpic_tuning {
     int32_t tile[3];            /* cells per tile edge, <= 64: divisors of n, or the default edge (the
-                                   last tile of an axis may then be shorter) */
+                                   last tile of an axis may then be shorter).  A default tile that
+                                   leaves the halo no room gives way to a smaller one */
     int32_t halo;               /* cells staged around a tile, 0..4 */
     int32_t split;              /* CTAs per (species, tile), 1..64; 0 (the default): chosen for each launch
                                    so that the CTAs fill the chip, up to 16 */

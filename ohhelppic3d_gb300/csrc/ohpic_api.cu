@@ -55,15 +55,6 @@ int64_t tiles_of(const int n[3], const int tile[3])
     return nt;
 }
 
-// The widest halo that a tile's staged box has room for; -1 when none.
-int halo_room(const ohpic_config &k, const int tile[3])
-{
-    Geom g;
-    int h = kMaxHalo;
-    while (h >= 0 && !make_geom(k, tile, h, g, tile)) --h;
-    return h;
-}
-
 // Default tile of a grid: edges of about 8 cells, or of about 4 along z, then y,
 // then x while the species' tiles are too few to occupy the chip (152 SMs, two
 // CTAs each).  FP32 push, tiles of 8 x 8 x 8 against the ones this rule takes,
@@ -71,15 +62,9 @@ int halo_room(const ohpic_config &k, const int tile[3])
 // ppc 49 -> 26 us (8 x 4 x 4), 32^3 x 16 ppc 49.6 -> 37.9 us (8 x 8 x 4); FP64 at
 // 32^3 353 -> 249 us.  From 48^3 on (432 tiles) 8 x 8 x 8 is as fast as any.
 // Two CTAs must fit an SM (boxes of at most pair_nodes nodes).
-// The halo may be widened later, and the caller may have given edges of the tile: the
-// open ones shrink until the box has the room that the largest powers of two dividing the
-// axes (at most 8) leave it.  Where those have no room for the halo, they stand, and the
-// shape is refused.  FP64 push, 16 ppc, two species, against the tiles before that rule,
-// which took no halo of 4: 45^3 (9,9,5) 331 us for (9,9,8) 343, 54^3 (9,9,6) 579 for
-// (9,9,8) 546, 63^3 (9,7,7) 818 for (9,9,8) 858, 90 x 60 x 30 (9,8,6) 595 for (9,8,8) 585.
 constexpr int64_t kFewTiles = 200;
 
-void default_tile(const ohpic_config &k, int halo, int tile[3])
+void default_tile(const ohpic_config &k, int tile[3])
 {
     const int n[3] = {k.nx, k.ny, k.nz};
     const int64_t pair_nodes = k.precision == OHPIC_FP64 ? 2580 : 3540;
@@ -91,38 +76,61 @@ void default_tile(const ohpic_config &k, int halo, int tile[3])
     }
     auto nodes = [&]() {
         int64_t v = 1;
-        for (int d = 0; d < 3; ++d) v *= tile[d] + 2 * halo + 1;
+        for (int d = 0; d < 3; ++d) v *= tile[d] + 2 * kDefaultHalo + 1;
         return v;
     };
     for (int d = 2; d >= 0 && nodes() > pair_nodes; --d)
         if (k.tile[d] <= 0) tile[d] = std::min(tile[d], want[d]);
+}
 
-    int plain[3];
+// True when a tile's staged box fits a CTA's shared memory.
+bool box_fits(const ohpic_config &k, const int tile[3], int halo)
+{
+    Geom g;
+    return make_geom(k, tile, halo, g, tile);
+}
+
+// The default tile for each halo.  The one of default_tile stands wherever its box fits.
+// Where it does not (the caller gave large edges for the others, or widens the halo) the
+// open edges shrink as far as the box needs, provided that the largest powers of two
+// dividing those axes (at most 8) leave it the room; otherwise the shape is refused.
+// (The rule for the wide halos applied to every grid costs speed where the halo stays at
+// its default: FP64 push, 16 ppc, two species, 54^3 in tiles of (9,9,6) for a halo of 4
+// 579 us, of (9,9,8) 546; 90 x 60 x 30 (9,8,6) 595, (9,8,8) 585.)
+void default_tiles(const ohpic_config &k, int tile[kMaxHalo + 1][3])
+{
+    const int n[3] = {k.nx, k.ny, k.nz};
+    int base[3], plain[3];
+    default_tile(k, base);
     for (int d = 0; d < 3; ++d) {
         plain[d] = k.tile[d] > 0 ? k.tile[d] : 8;
         while (k.tile[d] <= 0 && n[d] % plain[d]) plain[d] /= 2;
     }
-    const int room = halo_room(k, plain);
-    if (room < halo) std::copy(plain, plain + 3, tile);
-    while (halo_room(k, tile) < room) {
-        // the widest of the edges that leave a shorter last tile, else the widest, to the next
-        // one that divides the axis, or to one equal tile more
-        int at = -1, rank = -1;
-        for (int d = 2; d >= 0; --d) {
-            const int r = tile[d] + (n[d] % tile[d] ? 64 : 0);
-            if (k.tile[d] <= 0 && tile[d] > 1 && r > rank) {
-                at = d;
-                rank = r;
+    auto shrunk = [&](int halo, int t[3]) {
+        std::copy(base, base + 3, t);
+        while (!box_fits(k, t, halo) && box_fits(k, plain, halo)) {
+            // the widest of the edges that leave a shorter last tile, else the widest, to the
+            // next one that divides the axis, or to one equal tile more
+            int at = -1, rank = -1;
+            for (int d = 2; d >= 0; --d) {
+                const int r = t[d] + (n[d] % t[d] ? 64 : 0);
+                if (k.tile[d] <= 0 && t[d] > 1 && r > rank) {
+                    at = d;
+                    rank = r;
+                }
             }
+            const int w = t[at], more = (n[at] + w - 1) / w + 1;
+            t[at] = std::min(w - 1, (n[at] + more - 1) / more);
+            for (int e = w - 1; 2 * e >= w; --e)
+                if (n[at] % e == 0) {
+                    t[at] = e;
+                    break;
+                }
         }
-        const int t = tile[at], more = (n[at] + t - 1) / t + 1;
-        tile[at] = std::min(t - 1, (n[at] + more - 1) / more);
-        for (int e = t - 1; 2 * e >= t; --e)
-            if (n[at] % e == 0) {
-                tile[at] = e;
-                break;
-            }
-    }
+    };
+    shrunk(kDefaultHalo, tile[kDefaultHalo]);
+    std::copy(tile[kDefaultHalo], tile[kDefaultHalo] + 3, base);
+    for (int h = 0; h <= kMaxHalo; ++h) shrunk(h, tile[h]);
 }
 
 }  // namespace
@@ -563,11 +571,10 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     const int n[3] = {k.nx, k.ny, k.nz};
     for (int d = 0; d < 3; ++d)
         if (k.tile[d] > 0 && (n[d] % k.tile[d] != 0 || k.tile[d] > 64)) return OHPIC_ERR_INVALID;
-    constexpr int kHalo = 2;
-    int tile[3];
-    default_tile(k, kHalo, tile);
+    int tile[kMaxHalo + 1][3];
+    default_tiles(k, tile);
     Geom shape;
-    if (!make_geom(k, tile, kHalo, shape, tile)) return OHPIC_ERR_INVALID;
+    if (!make_geom(k, tile[kDefaultHalo], kDefaultHalo, shape, tile[kDefaultHalo])) return OHPIC_ERR_INVALID;
 
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || k.device < 0 || k.device >= ndev) {
@@ -584,7 +591,7 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
         return OHPIC_ERR_CUDA;
     }
 
-    c->halo = kHalo;
+    c->halo = kDefaultHalo;
     c->split = 0;
     c->with_energy = false;
     c->sc_dt = NAN;
@@ -594,10 +601,15 @@ int ohpic_create(const ohpic_config *cfg, ohpic_ctx **out)
     c->tma_polls = kTmaWaitPolls;
     Geom &g = c->g;
     g = shape;
-    for (int d = 0; d < 3; ++d) c->def_tile[d] = tile[d];
+    memcpy(c->def_tile, tile, sizeof(tile));
     // sort keys of any tile this context accepts: a tile edge divides its axis or
-    // is the default one, whose tiles cover at least the axis
-    const int64_t nkeys = std::max(g.nkeys, g.ncell);
+    // is a default one, whose tiles cover at least the axis
+    int64_t nkeys = 1;
+    for (int d = 0; d < 3; ++d) {
+        int most = n[d];
+        for (const auto &t : tile) most = std::max(most, (n[d] + t[d] - 1) / t[d] * t[d]);
+        nkeys *= most;
+    }
 
     int64_t off = 0;
     for (int s = 0; s < k.nspecies; ++s) {
@@ -1120,8 +1132,18 @@ int ohpic_set_tuning(ohpic_ctx *c, const ohpic_tuning *t)
                     "tuning: split 0..64, deposit 0..4, sort_every >= 0, lane_particles 2 or 4");
     if (t->sort_lead < 0 || t->sort_lead > 4096 || (t->sort_lead != 0 && c->cfg.precision != OHPIC_FP32))
         return fail(c, OHPIC_ERR_INVALID, "tuning: sort_lead 0..4096, nonzero only in the FP32 form");
+    // edges that need not divide the axis: the default ones; a default tile without room
+    // for the halo gives way to the halo's own
+    int tile[3], edge[3] = {0, 0, 0};
+    bool is_default = false;
+    for (const auto &def : c->def_tile) is_default = is_default || std::equal(def, def + 3, t->tile);
+    const bool give_way = is_default && t->halo >= 0 && t->halo <= kMaxHalo && !box_fits(c->cfg, t->tile, t->halo);
+    std::copy(give_way ? c->def_tile[t->halo] : t->tile, (give_way ? c->def_tile[t->halo] : t->tile) + 3, tile);
+    for (const auto &def : c->def_tile)
+        for (int d = 0; d < 3; ++d)
+            if (def[d] == tile[d]) edge[d] = tile[d];
     Geom g2;
-    if (!make_geom(c->cfg, t->tile, t->halo, g2, c->def_tile))
+    if (!make_geom(c->cfg, tile, t->halo, g2, edge))
         return fail(c, OHPIC_ERR_INVALID, "tuning: tile edges must divide the grid (<= 64) and the staged box fit");
     cudaSetDevice(c->dev);
     materialize_records(c);

@@ -28,6 +28,7 @@ namespace ohpic {
 
 constexpr int kSegAlign = 64;       // particles; keeps every species segment 256-B aligned
 constexpr int kMaxHalo = 4;
+constexpr int kDefaultHalo = 2;
 // FP32 push with four particles per lane: per-thread prefetch stage in shared memory
 // (7 arrays x 256 threads x 16 bytes).
 constexpr size_t kQuadStageBytes = 7 * 256 * 16;
@@ -290,7 +291,7 @@ struct ohpic_ctx {
     bool field_valid;
     int64_t steps;
     int split;                  // CTAs per (species, tile); 0: pick_split for each launch
-    int def_tile[3];            // tile the context was created with
+    int def_tile[ohpic::kMaxHalo + 1][3];   // default tile of each halo
     int halo;
     int dep_strategy;           // OHPIC_DEPOSIT_* for the FP32 warp deposit
     int lane_particles;         // FP32 push/deposit: particles per lane (2 or 4)

@@ -1,8 +1,10 @@
-"""What a context takes for a tile: an edge left open (0) gets a default, and the defaults
-leave at least the room that the largest powers of two dividing the axes (at most 8) leave.
+"""What a context takes for a tile: an edge left open (0) gets a default, which shrinks where
+the staged box needs it, at least to the room that the largest powers of two dividing the
+axes (at most 8) leave.
 
-So a configuration is accepted exactly when those edges' box fits a CTA's shared memory at
-the default halo, and a tuning may widen the halo as far as those edges allow."""
+So a configuration is accepted whenever those edges' box fits a CTA's shared memory at the
+default halo, and a tuning may widen the halo as far as those edges allow; where the default
+tile has the room, it stands."""
 import ctypes as C
 import random
 
@@ -47,11 +49,13 @@ def test_open_edges_are_refused_only_where_no_box_fits(ohpic):
     """The shape is judged before any CUDA call, so this holds on any host."""
     P = ohpic
     for n, tile, fp64 in _configurations():
-        if any(t and v % t for v, t in zip(n, tile)):
+        if any(t and v % t for v, t in zip(n, tile)) or not _fits([t or 1 for t in tile], 2, fp64):
             assert _create(P, n, tile, fp64) == P.ERR_INVALID, (n, tile, fp64)
-        elif n[0] * n[1] * n[2] < 1 << 21:
-            want = _fits(_plain(n, tile), 2, fp64)
-            assert (_create(P, n, tile, fp64) != P.ERR_INVALID) == want, (n, tile, fp64)
+        elif n[0] * n[1] * n[2] < 1 << 21 and _fits(_plain(n, tile), 2, fp64):
+            assert _create(P, n, tile, fp64) != P.ERR_INVALID, (n, tile, fp64)
+    # few tiles: the default is smaller than the powers of two, and fits where they do not
+    assert not _fits(_plain((64, 64, 64), (64, 0, 0)), 2, False)
+    assert _create(P, (64, 64, 64), (64, 0, 0), False) != P.ERR_INVALID
 
 
 @pytest.mark.gpu
@@ -67,8 +71,11 @@ def test_default_tiles_take_every_halo(ohpic, n, tile, fp64):
                                     precision=P.FP64 if fp64 else P.FP32, weights=P.WEIGHTS_STANDARD)) as ctx:
         ctx.init_particles([P.species_init(ppc, 1.0), P.species_init(ppc, 0.1)])
         start = [ctx.download(s) for s in range(2)]
+        first = ctx.get_tuning()["tile"]
         for halo in [h for h in range(5) if _fits(plain, h, fp64)]:
             ctx.set_tuning(halo=halo)
+            tile = ctx.get_tuning()["tile"]
+            assert _fits(tile, halo, fp64) and (tile == first or not _fits(first, halo, fp64))
             for s in range(2):
                 ctx.upload(s, {k: v for k, v in start[s].items() if k != "ids"})
             ctx.step(0.1, 3)
@@ -76,3 +83,7 @@ def test_default_tiles_take_every_halo(ohpic, n, tile, fp64):
             want = want or got
             assert all(np.array_equal(a, b) for a, b in zip(got, want)), halo
         assert halo >= 2
+        ctx.set_tuning(halo=2)                 # the smaller tile goes on being taken
+        assert ctx.get_tuning()["tile"] == tile
+        ctx.set_tuning(tile=first)
+        assert ctx.get_tuning()["tile"] == first
