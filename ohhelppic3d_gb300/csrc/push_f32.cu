@@ -1010,7 +1010,7 @@ static void launch_k(ohpic_ctx *c, void (*kernel)(TileArgs, P, const CUtensorMap
                      int64_t blocks, size_t smem, const P &parts)
 {
     if (blocks <= 0) return;
-    allow_tile_shared(kernel);
+    allow_tile_shared(c, kernel);
     // CTAs over ~96 KB pair up on an SM only with the whole shared-memory carveout
     if (smem > 96 * 1024)
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -1058,7 +1058,7 @@ void launch_tiled_f32(ohpic_ctx *c, const TileArgs &a, int mode, int64_t blocks,
             auto kernel = fix == 16  ? tiled_f32_rec<W, 16>
                           : fix == 8 ? tiled_f32_rec<W, 8>
                                      : tiled_f32_rec<W, 0>;
-            allow_tile_shared(kernel);
+            allow_tile_shared(c, kernel);
             if (smem > 96 * 1024)
                 cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared);

@@ -411,7 +411,7 @@ static void launch_k(ohpic_ctx *c, void (*kernel)(TileArgs, P), const TileArgs &
                      const P &parts)
 {
     if (blocks <= 0) return;
-    allow_tile_shared(kernel);
+    allow_tile_shared(c, kernel);
     kernel<<<(unsigned)blocks, 256, smem, c->stream>>>(a, parts);
     ++c->launches;
 }
