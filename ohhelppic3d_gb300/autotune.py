@@ -7,7 +7,8 @@ context filled by the device injector with the same particles per cell and
 physics as the run, so tuning never advances the caller's simulation.  The per-CTA work depends only on the tile and the plasma,
 not on the grid size, so large grids are tuned on a proxy grid (by default at
 most 128 x 128 x 64 cells) holding the same particles per cell; CTAs per tile
-only matter when the grid has few tiles, where the proxy is the grid itself.
+only matter when the grid has few tiles, where the proxy is the grid itself
+(elsewhere the library goes on choosing them for each launch).
 
 Search: from the library defaults, particles per lane, deposit reduction, sort
 lead (FP32), every (tile shape, halo) pair, deposit reduction, sort lead and
@@ -179,9 +180,9 @@ def tune(n, dt, b0, qm, q, capacity_per_cell, species, precision=FP32, weights=0
             descend("sort_lead", leads)
             descend("lane_particles", [2, 4])
         if not proxy or grid == tuple(n):
-            # (a proxy leaves the split to the library, which picks it per launch)
+            # (a proxy leaves the split to the library, which picks it per launch, up to 16)
             best = {**best, "split": 1}
-            descend("split", [1, 2, 4, 8])
+            descend("split", [1, 2, 3, 4, 6, 8, 12, 16])
         # sort cadence: per-step push time grows as particles drift out of their tiles
         sort_ms = _sort_ms(ctx)
         ctx.set_push_timing(True)

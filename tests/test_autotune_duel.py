@@ -77,3 +77,20 @@ def test_near_ties_meet_on_a_fresh_plasma_one_context_at_a_time(monkeypatch, pro
     seen = {tuple(tr["tile"]): tr["push_ms"] for tr in best["trials"][::-1]
             if tr["halo"] == 1 and tr["sort_lead"] == 0 and tr["deposit"] == P.DEPOSIT_LANES and tr["lane_particles"] == 4}
     assert cold or seen[(16, 8, 8)] > seen[(8, 8, 8)]
+
+
+class Few(Hot):
+    """A grid of few tiles: the more CTAs share a tile, the faster, up to the library's own most."""
+
+    def step(self, dt, n=1):
+        super().step(dt, n)
+        self.push_ms += n * self.timing * (16.0 / min(max(self.t["split"], 1), 16) - (self.t["split"] > 1))
+
+
+def test_split_search_reaches_the_librarys_most(monkeypatch):
+    Hot.alive = Hot.made = 0
+    monkeypatch.setattr(A, "_ctx", lambda cfg_kw, species, seed=(42, 4242): Few(cold=True))
+    monkeypatch.setattr(A, "_sort_ms", lambda ctx: 1.0)
+    best = A.tune(n=(16, 16, 16), dt=0.1, b0=(0, 0, 0.5), qm=[-1.0], q=[1.0], capacity_per_cell=[9.0], species=[None],
+                  steps=6, max_cadence=5)
+    assert best["split"] == 16
