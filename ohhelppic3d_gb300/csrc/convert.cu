@@ -215,9 +215,10 @@ int grid_for(int64_t n, int threads)
 // that is nearly empty, or that do not fill the first one, wastes the rest.  The
 // split with the least waves x (cost of one CTA) is taken, a CTA costing a fixed
 // part (its boxes, its first loads) and a part per particle, both measured:
-// FP32 18 us + 3.7 ns, FP64 8 us + 27 ns.  A push of 48^3 x 16 ppc in FP64 (432
-// tiles of 8 x 8 x 8) goes from 851 us unsplit to 695 us with two CTAs per tile;
-// 16^3 x 64 ppc from 1445 to 157 us.  A split leaves at least 256 particles to a CTA.
+// FP32 18 us + 3.7 ns, FP64 8 us + 27 ns.  A push of 48^3 x 16 ppc in FP64 (two
+// species, 432 tiles of 8 x 8 x 8) goes from 461 us unsplit to 390 us with two CTAs per
+// tile; 16^3 x 64 ppc from 781 to 98.6 us, in FP32 from 121 to 24.6 us.  A split leaves at
+// least 256 particles to a CTA.
 int pick_split(const ohpic_ctx *c)
 {
     const int64_t items = (int64_t)c->cfg.nspecies * c->g.ntile;
