@@ -31,10 +31,11 @@ enum Xform { XF_R2HC, XF_HC2R, XF_DCT1, XF_DST1, XF_DCT2, XF_DCT3, XF_DST2, XF_D
 
 constexpr int kMaxFolds = 9;      // of up to 4096 intervals, down to kFoldEnd
 constexpr int kFoldEnd = 16;
-// A prime factor of R costs 2 R operations an element: whole solves against cuFFT's
-// (three kinds of axis, us) 64x53x48 99-162 against 249-398, 96x67x64 234-411
-// against 261-496, 96x83x64 335-576 against 326-632, 96x101x64 410-746 against
-// 376-745.
+// A prime factor of R costs R operations an element: whole solves (periodic to mixed
+// kinds of axis, us) against cuFFT's, and in brackets with 2 R operations, on which the
+// line was drawn: 64x53x48 76-123 (98-166) against 250-342, 96x67x64 176-310 (233-423)
+// against 263-587, 201x67x67 462-876 (853-1599) against 632-1727; above the line, with
+// 2 R, 96x83x64 335-576 against 326-632, 96x101x64 410-746 against 376-745.
 constexpr int kMaxPrime = 67;
 
 struct SubFft {
