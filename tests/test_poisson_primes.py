@@ -1,6 +1,6 @@
-"""Blocks whose edges hold a large prime factor, where the bounded solve's own passes do 2 R
-operations an element for a factor R: they take no longer for a node than blocks with
-the next prime, which go through cuFFT as every block did before the passes."""
+"""Blocks whose edges hold a large prime factor R, which costs the bounded solve's own passes
+R operations an element: they take no longer for a node than blocks with the next prime,
+which go through cuFFT as every block did before the passes."""
 import pytest
 
 pytestmark = pytest.mark.gpu
