@@ -921,6 +921,19 @@ static void sort_tiles(ohpic_ctx *c, float h)
     }
 }
 
+// Whether the tiles fill the chip for the tile-local re-sort, which gives each of them one
+// CTA (four on each of 152 SMs).  Where they fill less than 56% of their waves, the sort
+// over global counters, which divides the particles evenly, is the faster one: a re-sort
+// of 2 x 64 ppc, tile-local against global counters (FP32, FP64, us): 120 tiles 422 / 270,
+// 689 / 492, 216 tiles 472 / 414, 944 / 856, 343 tiles 563 / 596, 1296 / 1302, 512 tiles
+// 703 / 831, 1818 / 1862, 640 tiles (two waves) 1080 / 1013, 2641 / 2315, 1728 tiles 2031 /
+// 2472, 5711 / 5959.
+static bool tiles_fill(int64_t ntile)
+{
+    constexpr int64_t kSlots = 152 * 4;
+    return 100 * ntile >= 56 * kSlots * ((ntile + kSlots - 1) / kSlots);
+}
+
 int sort_particles(ohpic_ctx *c)
 {
     const Geom &g = c->g;
@@ -935,7 +948,7 @@ int sort_particles(ohpic_ctx *c)
     const double dt = std::isfinite(c->sc_dt) ? c->sc_dt : c->cfg.dt;
     float h = f32 && c->sort_lead > 0 ? (float)(c->sort_lead * dt) : 0.f;
     if (!std::isfinite(h)) h = 0.f;   // no usable step yet: sort by the current cell
-    if (c->sorted && sizeof(uint32_t) * ((size_t)g.tile_cells + axes) <= kTileSortMaxShared) {
+    if (c->sorted && tiles_fill(g.ntile) && sizeof(uint32_t) * ((size_t)g.tile_cells + axes) <= kTileSortMaxShared) {
         sort_tiles(c, h);
         c->steps_since_sort = 0;
         return OHPIC_OK;

@@ -1,0 +1,53 @@
+"""Re-sorts by tiles and by global counters: which one runs depends on the number of tiles,
+the particles and fields do not."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(P, n, ppc, precision, nspecies=2, tile=(0, 0, 0), **tuning):
+    cap = int(np.prod(n)) * ppc + 64
+    ctx = P.PicContext(P.make_config(n=n, dt=0.1, b0=(0, 0.1, 0.5), qm=[-1.0, 0.01, -1.0][:nspecies],
+                                     q=[-1.0 / ppc, 1.0 / ppc, -0.1 / ppc][:nspecies], capacity=[cap] * nspecies,
+                                     precision=precision, weights=P.WEIGHTS_STANDARD, sort_every=0, tile=tile))
+    ctx.set_tuning(**tuning)
+    ctx.init_particles([P.species_init(ppc, 1.0, (0.0, 0.0, 2.0)) for _ in range(nspecies)])
+    return ctx
+
+
+@pytest.mark.parametrize("precision,lead", [("fp64", 0), ("fp32", 0), ("fp32", 3)])
+@pytest.mark.parametrize("n", [(34, 10, 1), (31, 11, 1), (32, 19, 1), (29, 21, 1), (40, 17, 1), (227, 3, 1)])
+def test_either_resort_gives_the_same_bits(ohpic, n, precision, lead):
+    """340, 341, 608, 609, 680 and 681 tiles of one cell, against the few of the default."""
+    P = ohpic
+    prec, out = P.FP64 if precision == "fp64" else P.FP32, []
+    for tile in ((1, 1, 1), (0, 0, 0)):
+        with _context(P, n, 6, prec, tile=tile, **({"sort_lead": lead} if lead else {})) as ctx:
+            for _ in range(4):
+                ctx.sort()
+                ctx.step(0.1, 3)
+            ctx.sort()
+            parts = [ctx.download(s) for s in range(2)]
+            out.append([ctx.field(k) for k in (P.RHO, P.EX)] + [p[k] for p in parts for k in sorted(p)])
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_few_large_tiles_sort_as_fast_as_many_small_ones(ohpic):
+    P = ohpic
+    best = []
+    for tile in ((0, 0, 0), (8, 2, 8)):       # 120 tiles, and 440
+        with _context(P, (40, 22, 64), 64, P.FP32, 3, tile) as ctx:
+            ctx.sort()
+            times = []
+            for _ in range(6):
+                ctx.step(0.1, 5)
+                ctx.synchronize()
+                t = time.perf_counter()
+                ctx.sort()
+                ctx.synchronize()
+                times.append(time.perf_counter() - t)
+            best.append(min(times))
+    assert best[0] <= 1.25 * best[1], best
